@@ -32,6 +32,15 @@ __device__ __forceinline__ void cfma_cj(cd& acc, cd a, cd b) {
   acc.y = fma(a.x, b.y, acc.y);
   acc.y = fma(-a.y, b.x, acc.y);
 }
+// D (16x8, 4 per lane) += A (16x8 row, 4 per lane) * B (8x8 col, 2 per lane) on the FP64 tensor
+// path.  Lane l holds g = l/4, t = l%4: A (g, t), (g+8, t), (g, t+4), (g+8, t+4); B (t, g),
+// (t+4, g); D (g, 2t), (g, 2t+1), (g+8, 2t), (g+8, 2t+1).
+__device__ __forceinline__ void dmma16(double (&d)[4], const double (&a)[4], const double (&b)[2]) {
+  asm("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+      "{%0, %1, %2, %3};\n"
+      : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
+}
 // 1 / z (complex reciprocal, scaled like Smith's algorithm to avoid overflow)
 __host__ __device__ __forceinline__ cd crecip(cd z) {
   double ar = fabs(z.x), ai = fabs(z.y);
@@ -110,8 +119,6 @@ struct Workspace;
 // Q (and R) of each problem; uses the workspace's QR scratch (V, tau, V^H V, T V1^H)
 int qr_launch(const QrProblem& p, Workspace* ws, cudaStream_t s);
 bool qr_supported(int m, int n);
-// true when one cluster factorises an m x n problem (batched problems run in one launch)
-bool qr_batch_supported(int m, int n);
 // thin SVD X = U diag(S) V^H by one-sided Jacobi (S on the host, descending)
 int svd_launch(int m, int n, const cd* X, int64_t x_r, int64_t x_c, cd* U, int64_t u_r, int64_t u_c, double* S,
                cd* V, int64_t v_r, int64_t v_c, Workspace* ws, cudaStream_t st);

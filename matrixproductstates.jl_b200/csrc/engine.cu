@@ -254,28 +254,17 @@ int op_update_lenv(mpsb_ctx* ctx, const cd* A0, const cd* AL, cd* env, int lead,
 // trailing GEMMs may split K) invalidates captured graphs
 int run_qr(mpsb_ctx* ctx, const QrProblem& p0) {
   QrProblem p = p0;
-  int loops = 1;
   if (ctx->batch > 1 && p.batch == 1) {
     p.x_b = ctx->stride_of(p.X);
     p.q_b = ctx->stride_of(p.Q);
     p.r_b = p.R ? ctx->stride_of(p.R) : 0;
-    if (qr_batch_supported(p.m, p.n)) p.batch = ctx->batch;
-    else loops = ctx->batch;   // shapes beyond one cluster: one copy after the other
+    p.batch = ctx->batch;
   }
   void* before = ctx->ws.qr.p;
   void* before_sk = ctx->ws.splitk.p;
   void* before_side = ctx->ws.qr_side_ws ? ctx->ws.qr_side_ws->splitk.p : nullptr;
-  int st = MPSB_OK;
-  for (int b = 0; b < loops && st == MPSB_OK; ++b) {
-    QrProblem q = p;
-    if (loops > 1) {
-      q.X += b * p.x_b;
-      q.Q += b * p.q_b;
-      if (q.R) q.R += b * p.r_b;
-    }
-    count_launch(&ctx->ws);
-    st = qr_launch(q, &ctx->ws, ctx->stream);
-  }
+  count_launch(&ctx->ws);
+  const int st = qr_launch(p, &ctx->ws, ctx->stream);
   void* after_side = ctx->ws.qr_side_ws ? ctx->ws.qr_side_ws->splitk.p : nullptr;
   if (ctx->ws.qr.p != before || ctx->ws.splitk.p != before_sk || after_side != before_side) ctx->ws_generation++;
   return st;

@@ -41,16 +41,6 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
-// D (16x8, 4 per lane) += A (16x8 row, 4 per lane) * B (8x8 col, 2 per lane).  Lane l holds
-// g = l/4, t = l%4: A (g, t), (g+8, t), (g, t+4), (g+8, t+4); B (t, g), (t+4, g);
-// D (g, 2t), (g, 2t+1), (g+8, 2t), (g+8, 2t+1).
-__device__ __forceinline__ void dmma16(double (&d)[4], const double (&a)[4], const double (&b)[2]) {
-  asm("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-      "{%0, %1, %2, %3};\n"
-      : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
-      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
-}
-
 template <bool A_MCONTIG, bool B_KCONTIG>
 __device__ __forceinline__ void load_tile(cd* As, cd* Bs, const cd* A, const cd* B, const Gemm& g,
                                           int m0, int n0, int k0, int tid) {

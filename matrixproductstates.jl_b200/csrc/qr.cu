@@ -27,25 +27,33 @@
 // algorithm with panels of NB columns.  Every exchange between CTAs is a *push*: the
 // producer writes its values straight into each consumer's shared memory with st.async,
 // whose completion is counted in bytes on the consumer's mbarrier; the consumer waits on
-// its own mbarrier (bounded) and then reads only local shared memory.  No cluster-wide
-// barrier sits inside the loops.
-//   * column j: each warp reduces its panel columns over the CTA's rows with warp shuffles
-//     (lane = row) and pushes the sums to all C CTAs; the owner of row j pushes that row;
-//     after the wait warp 0 forms the reflector, w = v^H A and the new column of the
-//     compact-WY factor T, and every warp updates its columns;
-//   * trailing columns: partials of V^H A pushed to the owner of each column slice,
-//     reduced there in a fixed order with T^H applied, the slice pushed to every CTA,
-//     then A -= V W locally.
-// The cluster kernel ends with R, the explicit reflectors V (m x n, unit lower trapezoidal)
-// and tau in global memory, and E = [I; 0] in Q.  Q is then formed on the whole GPU with the
-// UT-transform identity  Q = (I - V T V^H) E = E - V (T V1^H),  T^{-1} = diag(1/tau) +
-// striu(V^H V)  (V1 = top n x n block of V): a tensor-core GEMM for G = V^H V, one
-// back-substitution kernel for M = T V1^H (T^{-1} M = V1^H, so M[i,:] = tau_i (V1^H[i,:] -
-// sum_{k>i} G[i,k] M[k,:]) needs no division and gives M[i,:] = 0 when tau_i = 0), and a
-// tensor-core GEMM for Q -= V M.  In exact arithmetic this is zungqr's Q.
-// Reductions run in a fixed order, so every CTA computes bit-identical reflectors and
+// its own mbarrier (bounded) and then reads only local shared memory.
+//   * column j: the panel sits in the registers of four warps, four columns each (lane = row).
+//     Each forms conj(x)^T a for its columns over the CTA's rows and pushes the sums to all C CTAs;
+//     after the exchange each sums the ranks, forms the reflector for itself, updates its columns and
+//     the next column x.  The exchange is the only synchronisation of a column step: a hand-over
+//     between warps through shared memory costs 160 clocks, an exchange between CTAs about 400, the
+//     reflector about 200 (FP64 latency 8 clocks, a shuffle 24), so the redundant arithmetic is cheaper.
+//   * the compact-WY factor T of a panel is built by a ninth warp, a column behind.
+//   * block reflectors: partials of V^H A on the FP64 tensor path, one bulk copy to the owner of
+//     each column slice, reduced there in a fixed order with T (or T^H) applied, the slice copied to
+//     every CTA, then A -= V W on the tensor path.
+//   * Q = H(1)...H(n) [I; 0] is formed in place in shared memory by applying the panels' block
+//     reflectors backwards to E (zungqr), so the matrix is read once and Q written once.
+// Reductions run in a fixed order, so every CTA and warp computes bit-identical reflectors and
 // results are reproducible run to run.  Each wait gives up after a bounded number of polls,
 // records the timeout in the error word and lets the kernel run to completion.
+//
+// Shapes beyond one cluster (for example 2048 x 512) are factored in outer panels of up to 64
+// columns by the same kernel, with the trailing updates and Q as GEMMs (qr_blocked).
+//
+// What bounds it: the chain of column steps (512 x 128: 2350 clocks a step at 16 CTAs, 60 % of the
+// time, 4-6 clocks an instruction; 2140 at 4 CTAs, 1340 at one), then the products, which run at the
+// FP64 tensor rate of the cluster's SMs.  One row per lane and many CTAs beat more rows per lane
+// (512 x 128 at 1 / 2 / 4 rows: 254 / 324 / 491 us) because the products scale with the CTAs.
+// Against the form with a reflector warp behind block barriers, Q as GEMMs over a back substitution
+// and outer panels of 16 columns (B200, Q only): 64 x 32 108.7 -> 51.2 us, 512 x 128 394 -> 254,
+// 512 x 256 818 -> 677, 2048 x 512 3990 -> 2510.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -59,19 +67,30 @@ namespace cg = cooperative_groups;
 namespace mpsb {
 namespace {
 
-constexpr int NT = 256, NW = 8;
+constexpr int NB = 16;                 // panel width
+constexpr int CW = 4, NWP = NB / CW;   // panel columns per warp, warps that hold the panel
+constexpr int NWM = 8;                 // warps of the block reflectors' products
+constexpr int NT = 32 * (NWM + 1);     // and the warp that builds T
 constexpr int CMAX = 16;
 constexpr size_t SMEM_LIMIT = 227 * 1024;
-constexpr int WAIT_LIMIT = 1 << 22;
-enum { MB_COL0 = 0, MB_COL1, MB_RS, MB_AG, MB_COUNT };
+constexpr int WAIT_LIMIT = 1 << 20;
+constexpr int LDT = NB + 1, LDR = NB + 1, LDW = NB + 1;   // leading dimensions of T, the exchanged partials, the gathered W
+enum { MB_COL = 0, MB_RS = 2, MB_AG, MB_COUNT };
+constexpr int BAR_PANEL = 1, BAR_TILES = 2, BAR_END = 3;   // named barriers: a step (C == 1), the product warps, a panel's end
 
 struct QrParams {
   QrProblem p;
-  cd* V;     // [batch][n][m] explicit unit lower trapezoidal reflectors (output)
-  cd* Tg;    // [batch][npanels][NB][NB] compact-WY factor of every panel (output)
-  int C, npanels, ldS, ksmax;
+  // form_q: Q goes to p.Q and T is scratch, [batch][npanels][NB][NB].  Otherwise the explicit unit
+  // lower trapezoidal reflectors go to V (leading dimension v_ld) and the compact-WY factor of the
+  // whole matrix to T (n x n, leading dimension t_ld).
+  int form_q;
+  cd* V;
+  int64_t v_ld, v_b;
+  cd* T;
+  int64_t t_ld, t_b;
+  int C, npanels, ldS, nc, ksc;   // nc: columns per exchange of a block reflector, ksc = ceil(nc / C)
   // shared-memory offsets (complex elements) and the byte offset of the mbarriers
-  int o_S, o_rcol, o_rrs, o_w2s, o_rag, o_T, o_bc, o_tst, o_mbar;
+  int o_S, o_V, o_col, o_rcol, o_stg, o_rrs, o_w2s, o_w2o, o_rag, o_T, o_cst, o_tst, o_mbar;
 };
 
 // ---- PTX helpers -------------------------------------------------------------------
@@ -88,18 +107,41 @@ __device__ __forceinline__ void st_async(uint32_t raddr, cd v, uint32_t rmbar) {
   asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [%0], {%1, %2}, [%3];"
                ::"r"(raddr), "d"(v.x), "d"(v.y), "r"(rmbar) : "memory");
 }
+// bulk copy of this CTA's shared memory into a cluster CTA's, completion counted on its mbarrier
+__device__ __forceinline__ void bulk_push(uint32_t rdst, uint32_t src, uint32_t bytes, uint32_t rmbar) {
+  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(rdst), "r"(src), "r"(bytes), "r"(rmbar) : "memory");
+}
+__device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void mbar_init(uint32_t mbar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar), "r"(count) : "memory");
 }
 __device__ __forceinline__ void mbar_expect(uint32_t mbar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes) : "memory");
 }
+// whether the phase of the given parity has completed, after a hardware-bounded suspension
 __device__ __forceinline__ bool mbar_test(uint32_t mbar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
-      "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
       : "=r"(ok) : "r"(mbar), "r"(parity) : "memory");
   return ok != 0;
+}
+template <int ID, int THREADS>
+__device__ __forceinline__ void bar_sync() { asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(THREADS) : "memory"); }
+__device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
+}
+// Bounded wait of one warp on the phase of the given parity.
+__device__ __forceinline__ void warp_wait(uint32_t mbar, uint32_t parity, bool& failed, int* err) {
+  int it = 0;
+  while (!failed && !mbar_test(mbar, parity)) {
+    if (++it >= WAIT_LIMIT) {
+      failed = true;
+      if (err) atomicOr(err, 1);
+    }
+  }
+  __syncwarp();
 }
 // Bounded wait of the whole CTA on the phase of the given parity.  Only thread 0 polls --
 // polling warps would compete with the computing warps for the shared-memory pipe -- and the
@@ -119,18 +161,6 @@ __device__ __forceinline__ void cta_wait(uint32_t mbar, uint32_t parity, bool& f
   __syncthreads();
 }
 
-// sum of the C partials part[q*stride] in a fixed order (tree over the ranks, independent loads)
-__device__ __forceinline__ cd sum_ranks(const cd* part, int stride, int C) {
-  cd v[CMAX];
-#pragma unroll
-  for (int q = 0; q < CMAX; ++q) v[q] = (q < C) ? part[q * stride] : cmk(0.0, 0.0);
-#pragma unroll
-  for (int w = CMAX / 2; w > 0; w >>= 1)
-#pragma unroll
-    for (int q = 0; q < w; ++q) v[q] = cadd(v[q], v[q + w]);
-  return v[0];
-}
-
 // The exponent slot of a rank's column message: no nonzero entry below the diagonal.
 constexpr int ESENT = -100000;
 
@@ -148,8 +178,6 @@ __device__ __forceinline__ cd cscal(cd v, double f) { return cmk(v.x * f, v.y * 
 
 // Half-width of the binary-exponent window [2^-SWIN, 2^(SWIN+1)) inside which nothing is scaled.
 constexpr int SWIN = 256;
-constexpr double WHI = 0x1p256, WLO = 0x1p-256;   // 2^SWIN, 2^-SWIN
-static_assert(SWIN == 256, "WHI / WLO follow SWIN");
 
 // A CTA whose partials are those of x 2^-e sends its |x|^2 partial (real) in the imaginary
 // part and a quiet NaN carrying SCODE + e in the real part, so the unscaled combination of the
@@ -160,16 +188,16 @@ __device__ __forceinline__ double scale_nan(int e) {
 }
 __device__ __forceinline__ int scale_of_nan(double v) { return (int)((__double_as_longlong(v) & 0xffffll) - SCODE); }
 
-// The reflector when some rank scaled its partials or alpha lies outside the unit range (rare:
+// The reflector when x == 0, some rank scaled its partials or alpha lies outside the window (rare:
 // kept out of line so the common path's instructions stay the plain formula's).  Lane c < pw
-// of warp 0 gets s = its combined partial at the scale 2^-E (lane jl: |x|^2 at 2^-2E), and
+// of a warp gets s = its combined partial at the scale 2^-E (lane jl: |x|^2 at 2^-2E), and
 // every lane tau, beta, rs = 1/(alpha - beta) at 2^-E, and fE = 2^-E.  Returned by value, so
 // the caller's variables stay in registers on the common path.
 struct Reflector {
-  cd s, tau, beta, rs;
-  double fE;
+  cd s, tau, rs, xj;
+  double beta_x, beta_y, ib, fE;
 };
-__device__ __noinline__ Reflector reflector_scaled(const cd* rb, int RS, int C, int lane, int jl, int pw, cd alpha) {
+__device__ __noinline__ Reflector reflector_scaled(const cd* rb, int C, int lane, int jl, int pw, cd alpha) {
   Reflector o;
   int e[CMAX];
   int ex = ESENT;
@@ -177,7 +205,7 @@ __device__ __noinline__ Reflector reflector_scaled(const cd* rb, int RS, int C, 
   for (int q = 0; q < CMAX; ++q) {
     e[q] = ESENT;
     if (q < C) {
-      const cd pq = rb[q * RS + jl];
+      const cd pq = rb[q * NB + jl];
       e[q] = pq.x != pq.x ? scale_of_nan(pq.x) : (pq.x != 0.0 ? 0 : ESENT);
     }
     ex = max(ex, e[q]);
@@ -188,27 +216,34 @@ __device__ __noinline__ Reflector reflector_scaled(const cd* rb, int RS, int C, 
 #pragma unroll
     for (int q = 0; q < CMAX; ++q) {
       if (q >= C || e[q] == ESENT) continue;
-      cd pq = rb[q * RS + lane];
+      cd pq = rb[q * NB + lane];
       if (lane == jl) pq = cmk(pq.x != pq.x ? pq.y : pq.x, 0.0);
       v = cadd(v, cscal(pq, pow2neg(mult * (e[q] - ex))));
     }
   }
   const double xn2x = __shfl_sync(0xffffffffu, v.x, jl);   // |x|^2 2^-2ex
   const unsigned ha = (unsigned)__double2hiint(fmax(fabs(alpha.x), fabs(alpha.y)));
+  o.fE = 1.0;
+  o.s = v;
+  o.tau = cmk(0.0, 0.0); o.rs = cmk(1.0, 0.0); o.xj = cmk(0.0, 0.0); o.ib = 0.0;
+  o.beta_x = alpha.x; o.beta_y = alpha.y;
+  if (ex == ESENT && (alpha.y == 0.0 || ha == 0u)) return o;   // x == 0 and a real (or negligible) pivot: H = I
   int ea = expo_hi(ha);
   ea = (ha == 0u) ? ESENT : (ea >= -SWIN && ea <= SWIN ? 0 : ea);
-  const int E = max(ex, ea);   // not both ESENT: x == 0 with real alpha never gets here
+  const int E = max(ex, ea);
   o.fE = pow2i(-E);
   const cd as = cscal(alpha, o.fE);
   const double xn2 = (ex == ESENT) ? 0.0 : xn2x * pow2neg(2 * (ex - E));
   const double nrm = sqrt(as.x * as.x + as.y * as.y + xn2);
   const double b = -copysign(nrm, alpha.x);
   const double dr = as.x - b;
-  const double ib = 1.0 / b;
+  o.ib = 1.0 / b;
   const double id = 1.0 / (dr * dr + as.y * as.y);
-  o.tau = cmk((b - as.x) * ib, -as.y * ib);
-  o.beta = cmk(b * pow2i(E), 0.0);
+  o.tau = cmk((b - as.x) * o.ib, -as.y * o.ib);
+  o.beta_x = b * pow2i(E);
+  o.beta_y = 0.0;
   o.rs = cmk(dr * id, -as.y * id);
+  o.xj = cmk(dr, as.y);
   o.s = (ex == ESENT) ? cmk(0.0, 0.0) : cscal(v, pow2neg(ex - E));
   return o;
 }
@@ -216,73 +251,59 @@ __device__ __noinline__ Reflector reflector_scaled(const cd* rb, int RS, int C, 
 __device__ __forceinline__ cd shfl(cd v, int src) {
   return cmk(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
 }
-// ---- per-CTA shared memory map (complex elements) -------------------------------------
-// S     [(ROWS+1) * n]       this CTA's rows, column-major, ld = ROWS+1
-// rcol  [2][C][2*NB]         column exchange (two parities): pq from each rank, row j from its owner
-// rrs   [C][NB*ksmax]        partials of V^H A received from each rank for my column slice
-// w2s   [NB*ksmax]           my reduced slice
-// rag   [NB*n]               the gathered W2 (all slices)
-// T     [NB*NB]              compact-WY factor of the current panel (column-major NB x NB)
-// mbar  [MB_COUNT] u64
 
-// V[r, i] of panel p0 for global row g (unit lower trapezoidal, stored below the diagonal)
-#define VAL_V(g, i, rr) ((g) == p0 + (i) ? cmk(1.0, 0.0) : S[(p0 + (i)) * ldS + (rr)])
-
-// Partial sums W[i, k] = sum over this CTA's rows of conj(V[r, i]) A[r, kb + k] for the panel at
-// p0 (width pw), pushed with st.async to the owner of column slice k / KS.  Threads t in
-// [0, nthr) take (k, half panel) pairs; the rows of the panel's diagonal block (where V is 1 or
-// 0 above its stored part) are handled apart so the bulk loop carries no per-element tests.
-template <int ROWS, int NB>
-__device__ __forceinline__ void partials_push(const cd* S, int ldS, cd* rrs, uint32_t mb_rs, int crank, int ksmax,
-                                              int row0, int m, int p0, int pw, int kb, int nt, int KS, int t,
-                                              int nthr) {
-  const int lo = max(0, p0 - row0), hi = min(ROWS, m - row0);
-  const int mid = min(hi, max(lo, p0 + pw - row0));
-  for (int e = t; e < 2 * nt; e += nthr) {
-    const int k = e % nt, i0 = (e / nt) * (NB / 2);
-    const int iv = min(NB / 2, pw - i0);   // valid panel columns in this half
-    cd acc[NB / 2];
-#pragma unroll
-    for (int i = 0; i < NB / 2; ++i) acc[i] = cmk(0.0, 0.0);
-    const cd* Ak = S + (kb + k) * ldS;
-    for (int rr = lo; rr < mid; ++rr) {
-      const int g = row0 + rr;
-      const cd a = Ak[rr];
-#pragma unroll
-      for (int i = 0; i < NB / 2; ++i) {
-        const int ii = i0 + i;
-        if (i < iv && g >= p0 + ii) cfma_cj(acc[i], VAL_V(g, ii, rr), a);
-      }
-    }
-    for (int rr = mid; rr < hi; ++rr) {
-      const cd a = Ak[rr];
-#pragma unroll
-      for (int i = 0; i < NB / 2; ++i)
-        if (i < iv) cfma_cj(acc[i], S[(p0 + i0 + i) * ldS + rr], a);
-    }
-    const int so = k / KS, kk = k - so * KS;
-    const uint32_t rm = mapa(mb_rs, so);
-#pragma unroll
-    for (int i = 0; i < NB / 2; ++i)
-      if (i < iv) st_async(mapa(su32(&rrs[crank * NB * ksmax + (i0 + i) + NB * kk]), so), acc[i], rm);
-  }
+__device__ __forceinline__ double rsqrt_seed(double a) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+  return y;
+}
+__device__ __forceinline__ double rcp_seed(double a) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+  return y;
 }
 
-// Row `rr` of the panel's V (zero above its diagonal block and outside the matrix), in registers.
-template <int NB>
-__device__ __forceinline__ void load_vrow(cd (&v)[NB], const cd* S, int ldS, int rr, int g, int m, int p0, int pw) {
-#pragma unroll
-  for (int i = 0; i < NB; ++i)
-    v[i] = (i < pw && g >= p0 + i && g < m) ? VAL_V(g, i, rr) : cmk(0.0, 0.0);
+// The reflector of (alpha, x) with xn2 = |x|^2 (NaN: some rank scaled its partials), when xn2 and
+// alpha lie inside the window -- tested on the high words, beside the formula: 0 < xn2 < 2^1023 and
+// |Re alpha|, |Im alpha| < 2^SWIN; returns false otherwise.
+//   tau = (beta - alpha)/beta, rs = 1/(alpha - beta) = conj(alpha - beta)/|alpha - beta|^2 with
+//   |alpha - beta|^2 = |alpha|^2 + beta^2 + 2 |Re alpha| |beta|, xj = alpha - beta, ib = 1/beta
+// (beta carries the opposite sign of Re alpha, so nothing cancels).  It sits on the critical path of
+// every column, so |beta| = sqrt(n2), 1/|beta| and the reciprocal come from the hardware's 20-bit
+// seeds, the second taken from the first's unrefined value, and one third-order Newton-Raphson
+// (Householder) step each: errors below 2^-55 before the last rounding.
+__device__ __forceinline__ bool reflector(cd alpha, double xn2, Reflector& o) {
+  const unsigned hn = (unsigned)__double2hiint(xn2);
+  const unsigned ha = max((unsigned)__double2hiint(alpha.x) & 0x7fffffffu, (unsigned)__double2hiint(alpha.y) & 0x7fffffffu);
+  const bool in = hn - 0x00100000u < 0x7fe00000u - 0x00100000u && ha < (unsigned)(1023 + SWIN) << 20;
+  const double a2 = fma(alpha.x, alpha.x, alpha.y * alpha.y), ax2 = 2.0 * fabs(alpha.x);
+  const double n2 = a2 + xn2, s2 = a2 + n2;
+  const double y0 = rsqrt_seed(n2), n0 = n2 * y0;
+  const double z0 = rcp_seed(fma(ax2, n0, s2));
+  const double r = fma(-n0, y0, 1.0), p = fma(r, 0.375, 0.5);
+  const double y = fma(y0 * r, p, y0), nrm = fma(n0 * r, p, n0);
+  const double e = fma(-fma(ax2, nrm, s2), z0, 1.0);
+  const double z = fma(z0, fma(e, e, e), z0);
+  o.ib = -copysign(y, alpha.x);
+  o.beta_x = -copysign(nrm, alpha.x);
+  o.beta_y = 0.0;
+  o.tau = cmk(fma(-alpha.x, o.ib, 1.0), -alpha.y * o.ib);
+  o.xj = cmk(alpha.x - o.beta_x, alpha.y);
+  o.rs = cmk(o.xj.x * z, -alpha.y * z);
+  return in;
+}
+// a - f v
+__device__ __forceinline__ cd cfms(cd a, cd f, cd v) {
+  return cmk(fma(f.y, v.y, fma(-f.x, v.x, a.x)), fma(-f.y, v.x, fma(-f.x, v.y, a.y)));
 }
 
-template <int RPL, int NB>
+template <int RPL, bool SOLO>   // SOLO: a cluster of one CTA
 __global__ void __launch_bounds__(NT, 1) qr_kernel(QrParams P) {
-  constexpr int ROWS = 32 * RPL;
+  constexpr int ROWS = 32 * RPL, LDV = ROWS + 1;
   cg::cluster_group cluster = cg::this_cluster();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cd* sm = reinterpret_cast<cd*>(smem_raw);
-  const int C = P.C, ldS = P.ldS, ksmax = P.ksmax;
+  const int C = P.C, ldS = P.ldS, ksc = P.ksc;
   const int m = P.p.m, n = P.p.n;
   const int crank = (int)cluster.block_rank();
   const int prob = blockIdx.y;
@@ -291,456 +312,569 @@ __global__ void __launch_bounds__(NT, 1) qr_kernel(QrParams P) {
   int* err = P.p.err;
 
   cd* S = sm + P.o_S;
+  cd* Vs = sm + P.o_V;
+  cd* colbuf = sm + P.o_col;
   cd* rcol = sm + P.o_rcol;
+  cd* stg = sm + P.o_stg;
   cd* rrs = sm + P.o_rrs;
   cd* w2s = sm + P.o_w2s;
+  cd* w2o = sm + P.o_w2o;
   cd* rag = sm + P.o_rag;
-  cd* Tall = sm + P.o_T;
-  cd* bcs = sm + P.o_bc;        // tau, beta, 1/(alpha - beta) at scale 2^-E, and 2^-E of the current column
-  cd* bcw = bcs + 4;            // w_c of the current column
-  cd* tst = sm + P.o_tst;       // tst[jl*NB + c] = t_c (c < jl), tst[jl*NB + jl] = tau_jl
+  cd* Ts = sm + P.o_T;
+  cd* cst = sm + P.o_cst;
+  cd* tst = sm + P.o_tst;
+  cd* pst = tst + NB * NB;
   uint64_t* mb = reinterpret_cast<uint64_t*>(smem_raw + P.o_mbar);
-  uint32_t mbs[MB_COUNT];
-#pragma unroll
-  for (int k = 0; k < MB_COUNT; ++k) mbs[k] = su32(&mb[k]);
-  uint32_t ph[MB_COUNT];
-#pragma unroll
-  for (int k = 0; k < MB_COUNT; ++k) ph[k] = 0;
+  const uint32_t mb_rs = su32(&mb[MB_RS]), mb_ag = su32(&mb[MB_AG]);
+  uint32_t ph_rs = 0, ph_ag = 0;
   bool failed = false;
+  cd* Tg = P.T + (int64_t)prob * P.t_b;
 
   if (tid == 0) {
-#pragma unroll
-    for (int k = 0; k < MB_COUNT; ++k) mbar_init(mbs[k], 1);
+    for (int k = 0; k < 2; ++k) mbar_init(su32(&mb[MB_COL + k]), NWP + 1);
+    mbar_init(mb_rs, 1);
+    mbar_init(mb_ag, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  {  // ---- load this CTA's rows
+  {  // ---- load this CTA's rows, along whichever index is contiguous in X
     const cd* X = P.p.X + (int64_t)prob * P.p.x_b;
-    for (int e = tid; e < ROWS * n; e += NT) {
-      int rr = e % ROWS, cc = e / ROWS, g = row0 + rr;
-      S[cc * ldS + rr] = (g < m) ? X[(int64_t)g * P.p.x_r + (int64_t)cc * P.p.x_c] : cmk(0.0, 0.0);
+    if (P.p.x_c == 1 && P.p.x_r != 1) {
+      for (int e = tid; e < ROWS * n; e += NT) {
+        const int cc = e % n, rr = e / n, g = row0 + rr;
+        S[cc * ldS + rr] = (g < m) ? X[(int64_t)g * P.p.x_r + cc] : cmk(0.0, 0.0);
+      }
+    } else {
+      for (int e = tid; e < ROWS * n; e += NT) {
+        const int rr = e % ROWS, cc = e / ROWS, g = row0 + rr;
+        S[cc * ldS + rr] = (g < m) ? X[(int64_t)g * P.p.x_r + (int64_t)cc * P.p.x_c] : cmk(0.0, 0.0);
+      }
     }
+    if (!P.form_q && crank == 0)
+      for (int e = tid; e < n * n; e += NT) Tg[(e % n) + (int64_t)(e / n) * P.t_ld] = cmk(0.0, 0.0);
   }
   cluster.sync();   // mbarriers initialised cluster-wide before any push
 
+  // Columns kk in [0, ncols) -- columns 0 .. nprev-1 of the matrix, then cbase, cbase + 1, ... --
+  // get W = op(T) V^H A for the panel in Vs (rows >= p0, width pw), gathered in every CTA's rag, and
+  // all but the first nprev of them A -= V W.  op(T) = T^H in the factorisation, T for Q.
+  auto apply = [&](int p0, int pw, int nprev, int cbase, int ncols, bool factor) {
+    const int fg = lane >> 2, ft = lane & 3;
+    auto colp = [&](int kk) { return S + (kk < nprev ? kk : cbase + kk - nprev) * ldS; };
+    for (int c0 = 0; c0 < ncols; c0 += P.nc) {
+      const int ncc = min(P.nc, ncols - c0);
+      const int KS = (ncc + C - 1) / C, k0 = crank * KS, ks = max(0, min(ncc, k0 + KS) - k0);
+      const int ntile = (ncc + 7) / 8;
+      const bool active = row0 + ROWS > p0;
+      if (warp < NWM) {
+        // partials over this CTA's rows: 16 x 8 tiles, two per warp in flight
+        for (int t = warp; t < ntile; t += 2 * NWM) {
+          double re[2][4], im[2][4];
+          const bool two = t + NWM < ntile;
+#pragma unroll
+          for (int u = 0; u < 2; ++u)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) re[u][e] = im[u][e] = 0.0;
+          if (active) {
+            const cd* B0 = colp(c0 + min(8 * t + fg, ncc - 1));
+            const cd* B1 = colp(c0 + min(8 * (t + NWM) + fg, ncc - 1));
+#pragma unroll 2
+            for (int r = 0; r < ROWS; r += 8) {
+              // k index t <-> row 2t, t + 4 <-> row 2t + 1: odd leading dimensions then give the
+              // eight 16-byte loads of a quarter warp distinct banks
+              const int ra = r + 2 * ft;
+              double vr[4], vi[4], nvi[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const cd v = Vs[(fg + 8 * (e & 1)) * LDV + ra + (e >> 1)];
+                vr[e] = v.x; vi[e] = v.y; nvi[e] = -v.y;
+              }
+              const cd b00 = B0[ra], b01 = B0[ra + 1], b10 = B1[ra], b11 = B1[ra + 1];
+              const double br[2][2] = {{b00.x, b01.x}, {b10.x, b11.x}}, bi[2][2] = {{b00.y, b01.y}, {b10.y, b11.y}};
+#pragma unroll
+              for (int u = 0; u < 2; ++u)
+                if (u == 0 || two) {
+                  dmma16(re[u], vr, br[u]);
+                  dmma16(im[u], vr, bi[u]);
+                  dmma16(re[u], vi, bi[u]);
+                  dmma16(im[u], nvi, br[u]);
+                }
+            }
+          }
+#pragma unroll
+          for (int u = 0; u < 2; ++u)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const int i = fg + 8 * (e >> 1), kk = 8 * (t + u * NWM) + 2 * ft + (e & 1);
+              if (kk < ncc) stg[kk * LDR + i] = cmk(re[u][e], im[u][e]);
+            }
+        }
+        // each owner's slice of the partials, one bulk copy per rank (16-byte remote stores instead
+        // of these copies took 4 clocks each and set the time of the exchange)
+        fence_async();
+        bar_sync<BAR_TILES, 32 * NWM>();
+        if (warp == 0 && lane < C) {
+          const int q0 = lane * KS, nq = min(ncc, q0 + KS) - q0;
+          if (nq > 0)
+            bulk_push(mapa(su32(&rrs[crank * ksc * LDR]), lane), su32(&stg[q0 * LDR]), (uint32_t)(nq * LDR * sizeof(cd)),
+                      mapa(mb_rs, lane));
+        }
+      }
+      if (ks > 0) {
+        if (tid == 0) mbar_expect(mb_rs, (uint32_t)(C * LDR * ks * sizeof(cd)));
+        cta_wait(mb_rs, ph_rs, failed, err);
+        ph_rs ^= 1;
+      } else {
+        __syncthreads();
+      }
+      // the ranks' sum and op(T) W on my slice (zero beyond the panel width: V and T are), copied to
+      // every CTA; a column's 16 entries sit in one half warp
+      for (int e = tid; e < NB * ks; e += NT) {
+        const int i = e % NB, kk = e / NB;
+        const cd* src = rrs + kk * LDR + i;
+        cd w = cmk(0.0, 0.0);
+#pragma unroll 4
+        for (int q = 0; q < C; ++q) w = cadd(w, src[q * ksc * LDR]);
+        w2s[e] = w;
+        __syncwarp(__activemask());
+        const cd* t = factor ? Ts + LDT * i : Ts + i;
+        const int ts = factor ? 1 : LDT;
+        cd s0 = cmk(0.0, 0.0), s1 = cmk(0.0, 0.0);
+#pragma unroll 4
+        for (int i2 = 0; i2 < NB; i2 += 2) {
+          cd t0 = t[i2 * ts], t1 = t[(i2 + 1) * ts];
+          if (factor) { t0.y = -t0.y; t1.y = -t1.y; }
+          cfma(s0, t0, w2s[kk * NB + i2]);
+          cfma(s1, t1, w2s[kk * NB + i2 + 1]);
+        }
+        w2o[kk * LDW + i] = cadd(s0, s1);
+      }
+      fence_async();
+      __syncthreads();
+      if (warp == 0) {
+        if (lane == 0) mbar_expect(mb_ag, (uint32_t)(ncc * LDW * sizeof(cd)));
+        __syncwarp();
+        if (lane < C && ks > 0)
+          bulk_push(mapa(su32(&rag[k0 * LDW]), lane), su32(w2o), (uint32_t)(ks * LDW * sizeof(cd)), mapa(mb_ag, lane));
+      }
+      cta_wait(mb_ag, ph_ag, failed, err);
+      ph_ag ^= 1;
+      if (factor && !P.form_q && crank == 0 && c0 < nprev) {
+        // T[0:p0, panel] = -T[0:p0, 0:p0] (V_c^H V_p T_p), the bracket being the gathered W's ^H
+        const int kmax = min(nprev, c0 + ncc);   // the first nprev columns come in one chunk
+        for (int e = tid; e < kmax * pw; e += NT) {
+          const int i = e % kmax, jj = e / kmax;
+          cd s = cmk(0.0, 0.0);
+          for (int c = i; c < kmax; ++c) cfma_cj(s, rag[c * LDW + jj], Tg[i + (int64_t)c * P.t_ld]);
+          Tg[i + (int64_t)(p0 + jj) * P.t_ld] = cmk(-s.x, -s.y);
+        }
+      }
+      if (active && warp < NWM) {
+        for (int t = warp; t < ntile; t += NWM) {
+          if (c0 + 8 * t + 7 < nprev) continue;
+          double wr[2][2], wi[2][2];
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const int i = 8 * h + ft + 4 * e;
+              const cd w = rag[min(8 * t + fg, ncc - 1) * LDW + i];
+              wr[h][e] = w.x; wi[h][e] = w.y;
+            }
+          const int ka = 8 * t + 2 * ft;
+          cd* C0 = colp(c0 + min(ka, ncc - 1));
+          cd* C1 = colp(c0 + min(ka + 1, ncc - 1));
+          const bool ok0 = ka < ncc && c0 + ka >= nprev, ok1 = ka + 1 < ncc && c0 + ka + 1 >= nprev;
+#pragma unroll 2
+          for (int rb = 0; rb < ROWS; rb += 16) {
+            if (row0 + rb + 16 <= p0) continue;
+            double re[4], im[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const cd c = ((e & 1) ? C1 : C0)[rb + fg + 8 * (e >> 1)];
+              re[e] = c.x; im[e] = c.y;
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              double nvr[4], vi[4], nvi[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const cd v = Vs[(8 * h + ft + 4 * (e >> 1)) * LDV + rb + fg + 8 * (e & 1)];
+                nvr[e] = -v.x; vi[e] = v.y; nvi[e] = -v.y;
+              }
+              dmma16(re, nvr, wr[h]);
+              dmma16(im, nvr, wi[h]);
+              dmma16(re, vi, wi[h]);
+              dmma16(im, nvi, wr[h]);
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if ((e & 1) ? ok1 : ok0) ((e & 1) ? C1 : C0)[rb + fg + 8 * (e >> 1)] = cmk(re[e], im[e]);
+          }
+        }
+      }
+      __syncthreads();
+    }
+  };
+
   // ================================ factorisation ================================
-  int sp = 0;
+  // Two buffers of the exchange suffice: another CTA pushes step j + 2 after its exchange of step
+  // j + 1, so after every panel warp here pushed step j + 1, which each does when it has read step j.
+  int step = 0;   // column steps so far: buffers step & 1, phase parity (step / 2) & 1
+  const int rbuf = (C + 1) * NB;
+  const int pr = lane & 7, pc = CW * warp + (lane >> 3);   // this lane pushes column pc to ranks pr, pr + 8
+  const bool push0 = pr < C, push1 = pr + 8 < C;
+  uint32_t rd0, rd1, rm0, rm1;   // where: slot pc of this rank's row, and the exchange's mbarriers
+  {
+    const uint32_t slot = su32(rcol) + (uint32_t)(pc * sizeof(cd)), m0 = su32(&mb[MB_COL]);
+    rd0 = mapa(slot, push0 ? pr : 0); rm0 = mapa(m0, push0 ? pr : 0);
+    rd1 = mapa(slot, push1 ? pr + 8 : 0); rm1 = mapa(m0, push1 ? pr + 8 : 0);
+  }
+  const uint32_t off_sum = (uint32_t)(crank * NB * sizeof(cd)), off_piv = (uint32_t)(C * NB * sizeof(cd));
+  if (warp == NWM && lane == 0)   // the T warp's arrivals for the first two steps
+    for (int k = 0; k < 2; ++k) mbar_arrive(su32(&mb[MB_COL + k]));
   for (int pi = 0; pi < P.npanels; ++pi) {
     const int p0 = pi * NB;
     const int pw = min(NB, n - p0);
-    for (int jl = 0; jl < pw; ++jl) {
-      const int j = p0 + jl;
-      constexpr int RS = 2 * NB;   // per rank: NB sums, NB owner-row values
-      cd* rb = rcol + sp * (C * RS);
-      const uint32_t mbc = mbs[MB_COL0 + sp];
-      const int owner = j / ROWS;
-      // -- phase A: partial sums over this CTA's rows g > j, pushed to every CTA
-      cd x[RPL];
+    if (warp < NWP) {
+      const int cf = CW * warp;   // first column
+      cd a[CW][RPL], x[RPL];
 #pragma unroll
       for (int q = 0; q < RPL; ++q) {
-        int r = lane + 32 * q, g = row0 + r;
-        x[q] = (g > j && g < m) ? S[j * ldS + r] : cmk(0.0, 0.0);
-      }
-      {  // this warp's (at most two) panel columns c0 = warp, c1 = warp + NW, reduced together
-        static_assert(NB <= 2 * NW, "at most two panel columns per warp");
-        const int c0 = warp, c1 = warp + NW;
-        cd a0 = cmk(0.0, 0.0), a1 = cmk(0.0, 0.0);
-        double mx = 0.0;   // largest |Re|, |Im| of x over this CTA's rows (every warp finds the same)
+        const int r = lane + 32 * q;
+        x[q] = S[p0 * ldS + r];
 #pragma unroll
-        for (int q = 0; q < RPL; ++q) mx = fmax(mx, fmax(fabs(x[q].x), fabs(x[q].y)));
-        const unsigned hb = __reduce_max_sync(0xffffffffu, (unsigned)__double2hiint(mx));
-        auto partials = [&](const cd (&xv)[RPL]) {
+        for (int k = 0; k < CW; ++k) a[k][q] = cf + k < pw ? S[(p0 + cf + k) * ldS + r] : cmk(0.0, 0.0);
+        if (warp == 0) colbuf[ROWS + r] = a[1][q];   // column 1 for the step that follows column 0
+      }
+      for (int jl = 0; jl < pw; ++jl, ++step) {
+        const int j = p0 + jl, buf = step & 1;
+        cd* cs = cst + buf * 2 * NB;   // C == 1: the sums; the pivot row's entries in its owner
+        const uint32_t mbc = su32(&mb[MB_COL + buf]);
+        const int jr = j - row0;
+        const bool owner = jr >= 0 && jr < ROWS;
+#pragma unroll
+        for (int q = 0; q < RPL; ++q)
+          if (lane + 32 * q == jr) {
+#pragma unroll
+            for (int k = 0; k < CW; ++k) cs[NB + cf + k] = a[k][q];
+          }
+        __syncwarp();   // the pivot row's entries; and this warp's hand-over of column jl + 1, ordered by
+        if (!SOLO && lane == 0) {   // its arrival
+          if (warp == 0) mbar_expect(mbc, (uint32_t)((C + 1) * NB * sizeof(cd)));
+          else mbar_arrive(mbc);
+        }
+        // -- partial sums of conj(x) a over this CTA's rows g > j (x zero elsewhere)
+#pragma unroll
+        for (int q = 0; q < RPL; ++q)
+          if (row0 + lane + 32 * q <= j) x[q] = cmk(0.0, 0.0);
+        // the largest |Re|, |Im| of x over this CTA's rows, by the high words (every warp finds the same)
+        unsigned hx = 0;
+#pragma unroll
+        for (int q = 0; q < RPL; ++q)
+          hx = max(hx, max((unsigned)__double2hiint(x[q].x) & 0x7fffffffu, (unsigned)__double2hiint(x[q].y) & 0x7fffffffu));
+        const unsigned hb = __reduce_max_sync(0xffffffffu, hx);
+        // the scale 2^-e of this CTA's sums: none when x is 0 (or below 2^-1042) or its largest entry
+        // lies inside the window; else e is that entry's binary exponent, and the sums are redone on
+        // x 2^-e (a second round of the loop, so the rare case adds no code to the common one)
+        cd sum;
+        bool scaled = false;
+        cd xs[RPL];
+#pragma unroll
+        for (int q = 0; q < RPL; ++q) xs[q] = x[q];
+#pragma unroll 1
+        for (;;) {
+          cd sk[CW];
+#pragma unroll
+          for (int k = 0; k < CW; ++k) {
+            sk[k] = cmk(0.0, 0.0);
+#pragma unroll
+            for (int q = 0; q < RPL; ++q) cfma_cj(sk[k], xs[q], a[k][q]);
+          }
+          // lanes 8 k .. 8 k + 7 end with the sum of column cf + k
+          const bool lo = (lane & 16) == 0, lo2 = (lane & 8) == 0;
+          cd u0 = lo ? sk[0] : sk[2], u1 = lo ? sk[1] : sk[3];
+          const cd g0 = lo ? sk[2] : sk[0], g1 = lo ? sk[3] : sk[1];
+          u0.x += __shfl_xor_sync(0xffffffffu, g0.x, 16);
+          u0.y += __shfl_xor_sync(0xffffffffu, g0.y, 16);
+          u1.x += __shfl_xor_sync(0xffffffffu, g1.x, 16);
+          u1.y += __shfl_xor_sync(0xffffffffu, g1.y, 16);
+          sum = lo2 ? u0 : u1;
+          const cd give = lo2 ? u1 : u0;
+          sum.x += __shfl_xor_sync(0xffffffffu, give.x, 8);
+          sum.y += __shfl_xor_sync(0xffffffffu, give.y, 8);
+#pragma unroll
+          for (int off = 4; off > 0; off >>= 1) {
+            sum.x += __shfl_xor_sync(0xffffffffu, sum.x, off);
+            sum.y += __shfl_xor_sync(0xffffffffu, sum.y, off);
+          }
+          if (scaled || hb == 0u || hb - ((unsigned)(1023 - SWIN) << 20) < (unsigned)(2 * SWIN + 1) << 20) break;
+          scaled = true;
+          const double f = pow2i(-expo_hi(hb));
 #pragma unroll
           for (int q = 0; q < RPL; ++q) {
-            const int r = lane + 32 * q;
-            if (c0 < pw) {
-              const cd a = S[(p0 + c0) * ldS + r];
-              if (c0 == jl)     cfma_cj(a0, xv[q], xv[q]);   // |x|^2
-              else if (c0 > jl) cfma_cj(a0, xv[q], a);       // conj(x) a
-              else              cfma_cj(a0, a, xv[q]);       // conj(a) x  (V^H x for the T column)
-            }
-            if (c1 < pw) {
-              const cd a = S[(p0 + c1) * ldS + r];
-              if (c1 == jl)     cfma_cj(a1, xv[q], xv[q]);
-              else if (c1 > jl) cfma_cj(a1, xv[q], a);
-              else              cfma_cj(a1, a, xv[q]);
-            }
-          }
-        };
-        auto reduce = [&]() {
+            xs[q] = cscal(x[q], f);
 #pragma unroll
-          for (int off = 16; off > 0; off >>= 1) {
-            a0.x += __shfl_xor_sync(0xffffffffu, a0.x, off);
-            a0.y += __shfl_xor_sync(0xffffffffu, a0.y, off);
-            a1.x += __shfl_xor_sync(0xffffffffu, a1.x, off);
-            a1.y += __shfl_xor_sync(0xffffffffu, a1.y, off);
+            for (int k = 0; k < CW; ++k)   // column j's own copy, overwritten below, gives |x 2^-e|^2
+              if (cf + k == jl && row0 + lane + 32 * q > j) a[k][q] = xs[q];
           }
-        };
-        partials(x);
-        reduce();
-        // this CTA's scale 2^-e: e = 0 inside the window (the sums above stand), else mx's
-        // binary exponent, and the sums are redone on x 2^-e (ESENT: x == 0, or below 2^-1042)
-        const int ee = expo_hi(hb);
-        const int e_loc = (hb == 0u) ? ESENT : (ee >= -SWIN && ee <= SWIN ? 0 : ee);
-        if (e_loc != 0 && e_loc != ESENT) {
-          const double f = pow2i(-e_loc);
-          cd xs[RPL];
+        }
+        if (scaled && pc == jl) sum = cmk(scale_nan(expo_hi(hb)), sum.x);
+        // -- the exchange: every CTA gets all ranks' sums and the pivot row
+        const int c = lane & 15;
+        // this warp's columns, the pivot and the next; for one warp all, for T
+        const bool keeps = warp == (((jl >> 2) + 2) & 3), need = keeps || (c >> 2) == warp || c == jl || c == jl + 1;
+        const cd* rb = SOLO ? cs : rcol + buf * rbuf;
+        cd rv, s;
+        if (!SOLO) {
+          const uint32_t ob = (uint32_t)(buf * rbuf * sizeof(cd)), om = 8 * buf;
+          if (push0) st_async(rd0 + ob + off_sum, sum, rm0 + om);
+          if (push1) st_async(rd1 + ob + off_sum, sum, rm1 + om);
+          if (owner) {
+            const cd piv = cs[NB + pc];
+            if (push0) st_async(rd0 + ob + off_piv, piv, rm0 + om);
+            if (push1) st_async(rd1 + ob + off_piv, piv, rm1 + om);
+          }
+          warp_wait(mbc, (uint32_t)(step >> 1) & 1, failed, err);
+          const int h = (lane >> 4) * 8;   // lane c sums ranks 0 .. 7 of column c, lane c + 16 the others
+          rv = rb[C * NB + c];
+          cd part[8];
 #pragma unroll
-          for (int q = 0; q < RPL; ++q) xs[q] = cscal(x[q], f);
-          a0 = a1 = cmk(0.0, 0.0);
-          partials(xs);
-          reduce();
-        }
-        if (lane < C) {
-          const uint32_t rm = mapa(mbc, lane);
-          if (e_loc != 0 && e_loc != ESENT) {
-            if (c0 == jl) a0 = cmk(scale_nan(e_loc), a0.x);
-            if (c1 == jl) a1 = cmk(scale_nan(e_loc), a1.x);
-          }
-          if (c0 < pw) st_async(mapa(su32(&rb[crank * RS + c0]), lane), a0, rm);
-          if (c1 < pw) st_async(mapa(su32(&rb[crank * RS + c1]), lane), a1, rm);
-        }
-      }
-      if (crank == owner && warp == NW - 1 && lane < pw) {
-        const cd v = S[(p0 + lane) * ldS + (j - row0)];
-        for (int q = 0; q < C; ++q) st_async(mapa(su32(&rb[crank * RS + NB + lane]), q), v, mapa(mbc, q));
-      }
-      if (tid == 0) mbar_expect(mbc, (uint32_t)((C + 1) * pw * sizeof(cd)));
-      cta_wait(mbc, ph[MB_COL0 + sp], failed, err);
-      ph[MB_COL0 + sp] ^= 1;
-      // -- phase B: warp 0 forms the reflector from the gathered sums (local reads only) and
-      // publishes tau / beta / scale, w_c (c > jl) and t_c (c < jl, for T at panel end)
-      if (warp == 0) {
-        cd s = cmk(0.0, 0.0), rj = cmk(0.0, 0.0);
-        if (lane < pw) {
-          s = sum_ranks(rb + lane, RS, C);
-          rj = rb[owner * RS + NB + lane];
-        }
-        const cd alpha = shfl(rj, jl);
-        const double xn2 = __shfl_sync(0xffffffffu, s.x, jl);   // NaN: some rank scaled its partials
-        const double am = fabs(alpha.x) + fabs(alpha.y);   // alpha's window: (2^-SWIN, 2^SWIN)
-        cd tau, beta, rs;
-        double fE = 1.0;
-        if (xn2 == 0.0 && alpha.y == 0.0) {   // x == 0 (an unscaled nonzero x has |x|^2 >= 2^-2SWIN)
-          tau = cmk(0.0, 0.0); beta = alpha; rs = cmk(1.0, 0.0);
-        } else if (xn2 >= 0.0 && am < WHI && (xn2 > 0.0 || am > WLO)) {
-          // tau = (beta - alpha)/beta and rs = 1/(alpha - beta) from two independent
-          // reciprocals, 1/beta and 1/|alpha - beta|^2 (Re(alpha) - beta has no cancellation:
-          // beta carries the opposite sign of Re(alpha))
-          const double nrm = sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xn2);
-          const double b = -copysign(nrm, alpha.x);
-          const double dr = alpha.x - b;
-          const double ib = 1.0 / b;
-          const double id = 1.0 / (dr * dr + alpha.y * alpha.y);
-          tau = cmk((b - alpha.x) * ib, -alpha.y * ib);
-          beta = cmk(b, 0.0);
-          rs = cmk(dr * id, -alpha.y * id);
+          for (int q = 0; q < 8; ++q) part[q] = need && h + q < C ? rb[(h + q) * NB + c] : cmk(0.0, 0.0);
+#pragma unroll
+          for (int w = 4; w > 0; w >>= 1)
+#pragma unroll
+            for (int q = 0; q < w; ++q) part[q] = cadd(part[q], part[q + w]);
+          s = part[0];
+          s.x += __shfl_xor_sync(0xffffffffu, s.x, 16);
+          s.y += __shfl_xor_sync(0xffffffffu, s.y, 16);
         } else {
-          const Reflector o = reflector_scaled(rb, RS, C, lane, jl, pw, alpha);
-          s = o.s; tau = o.tau; beta = o.beta; rs = o.rs; fE = o.fE;
+          if (pr == 0) cs[pc] = sum;
+          bar_sync<BAR_PANEL, 32 * (NWP + 1)>();
+          s = cs[c];
+          rv = cs[NB + c];
         }
-        // w_c = a_c[j] + conj(rs) (x 2^-E)^H a_c and t_c = conj(V[j, c]) + rs V[:, c]^H (x 2^-E)
-        if (lane > jl && lane < pw) bcw[lane] = cadd(rj, cmul(cconj(rs), s));
-        else if (lane < jl) tst[jl * NB + lane] = cadd(cconj(rj), cmul(rs, s));
-        if (lane == 0) { bcs[0] = tau; bcs[1] = beta; bcs[2] = rs; bcs[3] = cmk(fE, 0.0); tst[jl * NB + jl] = tau; }
+        // -- the reflector, formed by every warp from the same sums
+        cd nx[RPL];   // column jl + 1 as updated by the reflectors before this one
+#pragma unroll
+        for (int q = 0; q < RPL; ++q) nx[q] = colbuf[((jl + 1) & 1) * ROWS + lane + 32 * q];
+        const cd alpha = shfl(rv, jl);
+        const double xn2 = __shfl_sync(0xffffffffu, s.x, jl);
+        Reflector o;
+        const bool plain = reflector(alpha, xn2, o);
+        if (__builtin_expect(!plain, 0)) {
+          o = reflector_scaled(rb, C, c, jl, pw, alpha);
+          s = o.s;
+#pragma unroll
+          for (int q = 0; q < RPL; ++q) {   // v = rs x 2^-E; column j is kept as v itself
+            x[q] = cscal(x[q], o.fE);
+#pragma unroll
+            for (int k = 0; k < CW; ++k)
+              if (cf + k == jl && row0 + lane + 32 * q > j) a[k][q] = cmul(o.rs, x[q]);
+          }
+        }
+        // lane c right of the pivot: a_c -= f v with f = conj(tau) (a_c[j] + conj(rs) x^H a_c) =
+        // conj(tau) a_c[j] - (x^H a_c)/beta and v = rs x, 1 at the pivot where x is set to 1/rs
+        const cd f = cmk(fma(o.tau.x, rv.x, fma(o.tau.y, rv.y, -o.ib * s.x)), fma(o.tau.x, rv.y, fma(-o.tau.y, rv.x, -o.ib * s.y)));
+        const cd hh = c > jl ? cmul(f, o.rs) : cmk(0.0, 0.0);
+        const cd hn = shfl(hh, min(jl + 1, NB - 1));
+        cd hk[CW];
+#pragma unroll
+        for (int k = 0; k < CW; ++k) hk[k] = shfl(hh, cf + k);
+        if (o.tau.x != 0.0 || o.tau.y != 0.0) {   // else H = I
+#pragma unroll
+          for (int q = 0; q < RPL; ++q) {
+            if (row0 + lane + 32 * q == j) x[q] = o.xj;
+#pragma unroll
+            for (int k = 0; k < CW; ++k) a[k][q] = cfms(a[k][q], hk[k], x[q]);
+            x[q] = cfms(nx[q], hn, x[q]);
+          }
+        } else {
+#pragma unroll
+          for (int q = 0; q < RPL; ++q) x[q] = nx[q];
+        }
+        if (keeps) {   // for T (see below) and the panel's end
+          if (lane <= jl) tst[jl * NB + lane] = lane == jl ? o.tau : cadd(rv, cmul(cconj(o.rs), s));
+          if (lane == 16) pst[jl] = plain ? o.rs : cmk(1.0, 0.0);
+          if (lane == 17) pst[NB + jl] = cmk(o.beta_x, o.beta_y);
+        }
+#pragma unroll
+        for (int k = 0; k < CW; ++k)
+          if (cf + k == jl + 2) {
+#pragma unroll
+            for (int q = 0; q < RPL; ++q) colbuf[(jl & 1) * ROWS + lane + 32 * q] = a[k][q];
+          }
       }
-      __syncthreads();
-      const cd tau = bcs[0], beta = bcs[1], rs = bcs[2];
-      const double fE = bcs[3].x;
-      if ((tau.x != 0.0) || (tau.y != 0.0)) {
-        cd vr[RPL];
+      // the panel back to shared memory, and its reflectors explicitly (unit lower trapezoidal): column
+      // c holds x below the pivot, v = pst[c] x (pst = 1 where v was kept)
+      bar_sync<BAR_END, 32 * (NWP + 1)>();
+#pragma unroll
+      for (int k = 0; k < CW; ++k) {
+        const int cc = cf + k;
+        const cd sc = pst[cc], beta = pst[NB + cc];
 #pragma unroll
         for (int q = 0; q < RPL; ++q) {
-          int g = row0 + lane + 32 * q;
-          vr[q] = (g == j) ? cmk(1.0, 0.0) : cmul(rs, fE == 1.0 ? x[q] : cscal(x[q], fE));   // x is 0 above j and in padding
-        }
-        const cd ctau = cconj(tau);
-        if (warp == (jl % NW)) {
-#pragma unroll
-          for (int q = 0; q < RPL; ++q) {
-            int r = lane + 32 * q, g = row0 + r;
-            if (g == j) S[j * ldS + r] = beta;
-            else if (g > j && g < m) S[j * ldS + r] = vr[q];
-          }
-        }
-        for (int c = warp; c < pw; c += NW) {
-          if (c > jl) {
-            const cd f = cmul(ctau, bcw[c]);
-#pragma unroll
-            for (int q = 0; q < RPL; ++q) {
-              int r = lane + 32 * q, g = row0 + r;
-              if (g >= j && g < m) {
-                cd* a = &S[(p0 + c) * ldS + r];
-                *a = csub(*a, cmul(f, vr[q]));
-              }
-            }
-          }
+          const int r = lane + 32 * q, g = row0 + r;
+          const cd v = cmul(sc, a[k][q]);
+          if (cc < pw) S[(p0 + cc) * ldS + r] = g < p0 + cc ? a[k][q] : (g == p0 + cc ? beta : v);
+          Vs[cc * LDV + r] = (cc >= pw || g < p0 + cc) ? cmk(0.0, 0.0) : (g == p0 + cc ? cmk(1.0, 0.0) : v);
         }
       }
-      __syncthreads();
-      sp ^= 1;
-    }
-    cd* Tp = Tall;   // the previous panel's T was last read before its all-gather wait
-    // T (compact WY, zlarft forward/columnwise) from the stashed t vectors, by warp 0 while the
-    // other warps start on the trailing partials: T[0:jl, jl] = -tau_jl T[0:jl, 0:jl] t_jl
-    if (warp == 0) {
-      for (int jl = 0; jl < pw; ++jl) {
-        const cd tj = tst[jl * NB + jl];
-        cd a4[4] = {cmk(0.0, 0.0), cmk(0.0, 0.0), cmk(0.0, 0.0), cmk(0.0, 0.0)};
-#pragma unroll
-        for (int c = 0; c < NB; ++c)   // T[lane, c] = 0 for c < lane, so c starts at 0 harmlessly
-          if (c < jl && lane < jl) cfma(a4[c & 3], Tp[lane + NB * c], tst[jl * NB + c]);
-        const cd acc = cadd(cadd(a4[0], a4[1]), cadd(a4[2], a4[3]));
-        if (lane < NB) Tp[lane + NB * jl] = (lane < jl) ? cmul(cmk(-tj.x, -tj.y), acc) : (lane == jl ? tj : cmk(0.0, 0.0));
+    } else if (warp == NWM) {
+      // T (compact WY, zlarft forward/columnwise), each column while the panel warps are at the next:
+      // T[0:jl, jl] = -tau_jl T[0:jl, 0:jl] t_jl with t_c = conj(pst[c] (a_c[j] + conj(rs) x^H x_c)),
+      // the bracket kept in tst; zero outside the panel width.  Lane i and i + 16 have row i, half of
+      // the sum each.
+      const int i = lane & 15, h = lane >> 4;
+      if (SOLO) bar_sync<BAR_PANEL, 32 * (NWP + 1)>();
+      for (int jl = 0; jl < NB; ++jl) {
+        // step jl's values are in place once every panel warp is at step jl + 1 or at the panel's end
+        if (jl + 1 < pw) {
+          if (SOLO) bar_sync<BAR_PANEL, 32 * (NWP + 1)>();
+          else warp_wait(su32(&mb[MB_COL + ((step + 1) & 1)]), (uint32_t)((step + 1) >> 1) & 1, failed, err);
+        } else if (jl + 1 == pw) {
+          bar_sync<BAR_END, 32 * (NWP + 1)>();
+        }
+        cd acc = cmk(0.0, 0.0), tau = cmk(0.0, 0.0);
+        if (jl < pw) {
+          tau = tst[jl * NB + jl];
+          for (int c = h; c < jl; c += 2) cfma(acc, Ts[i + LDT * c], cconj(cmul(pst[c], tst[jl * NB + c])));   // T[i, c] = 0 for c < i
+        }
+        acc.x += __shfl_xor_sync(0xffffffffu, acc.x, 16);
+        acc.y += __shfl_xor_sync(0xffffffffu, acc.y, 16);
+        const cd t = i == jl ? tau : (i < jl ? cmul(cmk(-tau.x, -tau.y), acc) : cmk(0.0, 0.0));
         __syncwarp();
-      }
-      if (crank == 0 && lane < NB) {   // lane-owned entries of T, zero outside the panel width
-        cd* Tout = P.Tg + ((int64_t)prob * P.npanels + pi) * NB * NB;
-        for (int jl = 0; jl < NB; ++jl)
-          Tout[lane + NB * jl] = (lane < pw && jl < pw) ? Tp[lane + NB * jl] : cmk(0.0, 0.0);
-      }
-    }
-
-    // -- trailing update A_t := (I - V T^H V^H) A_t
-    const int nt = n - p0 - pw;
-    if (nt > 0) {
-      const int kb = p0 + pw;
-      const int KS = (nt + C - 1) / C;
-      const int k0 = crank * KS, ks_mine = max(0, min(nt, k0 + KS) - k0);
-      // partials W[i, k] = sum_{my rows} conj(V[r, i]) A[r, k], pushed to the slice owner of k
-      if (warp > 0) partials_push<ROWS, NB>(S, ldS, rrs, mbs[MB_RS], crank, ksmax, row0, m, p0, pw, kb, nt, KS,
-                                            tid - 32, NT - 32);
-      __syncthreads();   // T complete before W2 = T^H W
-      if (tid == 0) mbar_expect(mbs[MB_RS], (uint32_t)(C * pw * ks_mine * sizeof(cd)));
-      cta_wait(mbs[MB_RS], ph[MB_RS], failed, err);
-      ph[MB_RS] ^= 1;
-      for (int e = tid; e < pw * ks_mine; e += NT) {
-        const int i = e % pw, kk = e / pw;
-        cd s = cmk(0.0, 0.0);
-        s = sum_ranks(rrs + i + NB * kk, NB * ksmax, C);
-        w2s[i + NB * kk] = s;
-      }
-      __syncthreads();
-      // W2 = T^H W on my slice, pushed to every CTA
-      for (int e = tid; e < pw * ks_mine; e += NT) {
-        const int i = e % pw, kk = e / pw;
-        cd s = cmk(0.0, 0.0);
-        for (int i2 = 0; i2 <= i; ++i2) cfma_cj(s, Tp[i2 + NB * i], w2s[i2 + NB * kk]);
-        const uint32_t la = su32(&rag[i + NB * (k0 + kk)]);
-        for (int q = 0; q < C; ++q) st_async(mapa(la, q), s, mapa(mbs[MB_AG], q));
-      }
-      if (tid == 0) mbar_expect(mbs[MB_AG], (uint32_t)(pw * nt * sizeof(cd)));
-      cta_wait(mbs[MB_AG], ph[MB_AG], failed, err);
-      ph[MB_AG] ^= 1;
-      // A[r, k] -= sum_i V[r, i] W2[i, k]: thread = (row, column group), its V row in registers
-      {
-        constexpr int G = NT / ROWS;
-        const int rr = tid % ROWS, grp = tid / ROWS, g = row0 + rr;
-        if (g >= p0 && g < m) {
-          cd v[NB];
-          load_vrow<NB>(v, S, ldS, rr, g, m, p0, pw);
-          for (int k = grp; k < nt; k += G) {
-            cd acc = cmk(0.0, 0.0);
-#pragma unroll
-            for (int i = 0; i < NB; ++i)
-              if (i < pw) cfma(acc, v[i], rag[i + NB * k]);
-            cd* a = &S[(kb + k) * ldS + rr];
-            *a = csub(*a, acc);
+        if (h == 0) {
+          Ts[i + LDT * jl] = t;
+          if (crank == 0 && i < pw && jl < pw) {
+            if (P.form_q) Tg[(int64_t)pi * NB * NB + i + NB * jl] = t;
+            else Tg[p0 + i + (int64_t)(p0 + jl) * P.t_ld] = t;
           }
         }
+        __syncwarp();
+        if (jl < pw) {   // its arrival for step + 2: the exchanges stay within two steps of this warp
+          if (!SOLO && lane == 0) mbar_arrive(su32(&mb[MB_COL + (step & 1)]));
+          ++step;
+        }
       }
-      __syncthreads();
+    } else {
+      step += pw;
     }
+    __syncthreads();
+    const int nprev = P.form_q ? 0 : p0, nt = n - p0 - pw;
+    if (nprev + nt > 0) apply(p0, pw, nprev, p0 + pw, nprev + nt, true);
   }
+  __syncthreads();
 
   // ---- optional R (rows < n)
   if (P.p.R) {
     cd* Rout = P.p.R + (int64_t)prob * P.p.r_b;
     for (int e = tid; e < ROWS * n; e += NT) {
-      int rr = e % ROWS, k = e / ROWS, g = row0 + rr;
+      const int rr = e % ROWS, k = e / ROWS, g = row0 + rr;
       if (g >= n) continue;
       Rout[(int64_t)g * P.p.r_r + (int64_t)k * P.p.r_c] = (k >= g) ? S[k * ldS + rr] : cmk(0.0, 0.0);
     }
   }
-  {  // ---- V (unit lower trapezoidal, explicit), tau, and E = [I; 0] into Q (this CTA's rows)
-    cd* V = P.V + (int64_t)prob * m * n;
-    cd* Q = P.p.Q + (int64_t)prob * P.p.q_b;
+  if (!P.form_q) {
+    cd* V = P.V + (int64_t)prob * P.v_b;
     for (int e = tid; e < ROWS * n; e += NT) {
-      int rr = e % ROWS, cc = e / ROWS, g = row0 + rr;
-      if (g >= m) continue;
-      V[g + (int64_t)cc * m] = g < cc ? cmk(0.0, 0.0) : (g == cc ? cmk(1.0, 0.0) : S[cc * ldS + rr]);
-      Q[(int64_t)g * P.p.q_r + (int64_t)cc * P.p.q_c] = cmk(g == cc ? 1.0 : 0.0, 0.0);
+      const int rr = e % ROWS, cc = e / ROWS, g = row0 + rr;
+      if (g < m) V[g + (int64_t)cc * P.v_ld] = g < cc ? cmk(0.0, 0.0) : (g == cc ? cmk(1.0, 0.0) : S[cc * ldS + rr]);
+    }
+    cluster.sync();   // no CTA leaves while a peer may still address its shared memory
+    return;
+  }
+  cluster.sync();   // rank 0's T of every panel
+
+  // ================================ Q = H(1) ... H(n) E ================================
+  cd tp = cmk(0.0, 0.0);   // an entry of the panel's T (zero outside its width)
+  if (tid < NB * NB) {
+    const int pw = n - (P.npanels - 1) * NB;
+    if (tid % NB < pw && tid / NB < pw) tp = __ldcg(&Tg[(int64_t)(P.npanels - 1) * NB * NB + tid]);
+  }
+  for (int pi = P.npanels - 1; pi >= 0; --pi) {
+    const int p0 = pi * NB, pw = min(NB, n - p0);
+    // the panel's reflectors to Vs, its columns of E to S (the later columns hold Q so far)
+    for (int e = tid; e < ROWS * NB; e += NT) {
+      const int rr = e % ROWS, i = e / ROWS, g = row0 + rr;
+      cd* a = S + (p0 + i) * ldS + rr;
+      Vs[i * LDV + rr] = (i >= pw || g < p0 + i) ? cmk(0.0, 0.0) : (g == p0 + i ? cmk(1.0, 0.0) : *a);
+      if (i < pw) *a = cmk(g == p0 + i ? 1.0 : 0.0, 0.0);
+    }
+    if (tid < NB * NB) Ts[tid % NB + LDT * (tid / NB)] = tp;
+    if (tid < NB * NB && pi > 0) tp = __ldcg(&Tg[(int64_t)(pi - 1) * NB * NB + tid]);   // in flight during this panel
+    __syncthreads();
+    apply(p0, pw, 0, p0, n - p0, false);
+  }
+  {
+    cd* Q = P.p.Q + (int64_t)prob * P.p.q_b;
+    if (P.p.q_c == 1 && P.p.q_r != 1) {
+      for (int e = tid; e < ROWS * n; e += NT) {
+        const int cc = e % n, rr = e / n, g = row0 + rr;
+        if (g < m) Q[(int64_t)g * P.p.q_r + cc] = S[cc * ldS + rr];
+      }
+    } else {
+      for (int e = tid; e < ROWS * n; e += NT) {
+        const int rr = e % ROWS, cc = e / ROWS, g = row0 + rr;
+        if (g < m) Q[(int64_t)g * P.p.q_r + (int64_t)cc * P.p.q_c] = S[cc * ldS + rr];
+      }
     }
   }
-  // no CTA leaves while a peer may still address its shared memory
-  cluster.sync();
+  cluster.sync();   // no CTA leaves while a peer may still address its shared memory
 }
-#undef VAL_V
 
 typedef void (*QrKernel)(QrParams);
 
-template <int NB>
-QrKernel kernel_rpl(int rpl) {
+QrKernel kernel_for(int rpl, int C) {
   switch (rpl) {
-    case 1: return qr_kernel<1, NB>;
-    case 2: return qr_kernel<2, NB>;
-    case 4: return qr_kernel<4, NB>;
+    case 1: return C == 1 ? qr_kernel<1, true> : qr_kernel<1, false>;
+    case 2: return C == 1 ? qr_kernel<2, true> : qr_kernel<2, false>;
+    case 4: return C == 1 ? qr_kernel<4, true> : qr_kernel<4, false>;
     default: return nullptr;
   }
 }
 
-QrKernel kernel_for(int rpl, int nb) {
-  if (nb == 16) return kernel_rpl<16>(rpl);
-  if (nb == 8) return kernel_rpl<8>(rpl);
-  if (nb == 4) return kernel_rpl<4>(rpl);
-  return nullptr;
-}
-
-size_t layout(QrParams& P, int n, int C, int rows, int nb) {
+size_t layout(QrParams& P, int n, int C, int rows, int nc) {
   P.C = C;
-  P.npanels = (n + nb - 1) / nb;
+  P.npanels = (n + NB - 1) / NB;
   P.ldS = rows + 1;
-  P.ksmax = (n + C - 1) / C;
+  P.nc = nc;
+  P.ksc = (nc + C - 1) / C;
   int o = 0;
   P.o_S = o;     o += P.ldS * n;
-  P.o_rcol = o;  o += 2 * C * 2 * nb;
-  P.o_rrs = o;   o += C * nb * P.ksmax;
-  P.o_w2s = o;   o += nb * P.ksmax;
-  P.o_rag = o;   o += nb * n;
-  P.o_T = o;     o += nb * nb;
-  P.o_bc = o;    o += 4 + nb;        // tau, beta, rs, 2^-E; w[nb]
-  P.o_tst = o;   o += nb * nb;       // t vectors (and tau) of the panel's columns
+  P.o_V = o;     o += (rows + 1) * NB;
+  P.o_col = o;   o += 2 * rows;
+  P.o_rcol = o;  o += 2 * (C + 1) * NB;
+  P.o_stg = o;   o += nc * LDR;
+  P.o_rrs = o;   o += C * P.ksc * LDR;
+  P.o_w2o = o;   o += P.ksc * LDW;
+  P.o_rag = o;   o += nc * LDW;
+  P.o_T = o;     o += NB * LDT;
+  P.o_cst = P.o_w2s = o;   o += std::max(4, P.ksc) * NB;   // column steps / block reflectors
+  P.o_tst = o;   o += NB * NB + 2 * NB;   // and per column the factor of x to v, and beta
   P.o_mbar = o * (int)sizeof(cd);
   return (size_t)P.o_mbar + MB_COUNT * sizeof(uint64_t);
 }
 
-// ---- M = T V1^H by block back substitution over the panels.  T^{-1} = diag(1/tau) +
-// striu(V^H V) is block upper triangular and its diagonal blocks are the inverses of the
-// panels' compact-WY factors T_p, so with G = V^H V and B = V1^H (upper triangular):
-//   M_p = T_p (B_p - sum_{q > p} G_pq M_q),  p = last panel .. 0.
-// One warp per column c of M (M is upper triangular: rows <= c), lanes over rows
-// (r = lane + 32 q), holding y = B[:, c] minus the updates so far.  Per panel: the panel's
-// rows of y are broadcast by shuffles, M_p = T_p y_p lands in the lanes of those rows, and
-// y -= G[:, panel] M_p updates the rows above.  The needed columns of G are staged in shared
-// memory one panel ahead (cp.async, double-buffered); the panels' T_p are staged once.
-constexpr int TR_WARPS = 8;
-
-template <int QMAX, bool STAGE>
-__global__ void __launch_bounds__(32 * TR_WARPS) qr_tmat_kernel(int m, int n, int nb, const cd* __restrict__ Vg,
-                                                                 const cd* __restrict__ Tg,
-                                                                 const cd* __restrict__ Gg, cd* __restrict__ Mg) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  cd* Gs = reinterpret_cast<cd*>(smem_raw);   // [2][nb][n]
-  cd* Ts = Gs + 2 * nb * n;                    // [npan][nb][nb]
-  const int prob = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int npan = (n + nb - 1) / nb;
-  const cd* V = Vg + (int64_t)prob * m * n;
-  const cd* T = Tg + (int64_t)prob * npan * nb * nb;
-  const cd* G = Gg + (int64_t)prob * n * n;
-  cd* M = Mg + (int64_t)prob * n * n;
-  const int c = blockIdx.x * TR_WARPS + warp;
-  const int ctop = min(n, (blockIdx.x + 1) * TR_WARPS) - 1;   // highest column in this CTA
-
-  cd y[QMAX];
-#pragma unroll
-  for (int q = 0; q < QMAX; ++q) {
-    const int r = lane + 32 * q;
-    y[q] = (c < n && r <= c) ? cconj(V[c + (int64_t)r * m]) : cmk(0.0, 0.0);
-  }
-  if (c < n)   // panels wholly below row c stay zero
-    for (int i = (c / nb + 1) * nb + lane; i < n; i += 32) M[i + (int64_t)c * n] = cmk(0.0, 0.0);
-
-  auto stage = [&](int pi, int buf) {   // G[r, p0 + j], r < p0, j < pw
-    if constexpr (!STAGE) return;
-    const int p0 = pi * nb, pw = min(nb, n - p0);
-    cd* dst = Gs + buf * nb * n;
-    for (int e = threadIdx.x; e < pw * p0; e += blockDim.x) {
-      const int r = e % p0, jj = e / p0;
-      const unsigned sa = static_cast<unsigned>(__cvta_generic_to_shared(dst + jj * n + r));
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(G + r + (int64_t)(p0 + jj) * n));
-    }
-    asm volatile("cp.async.commit_group;\n" ::);
-  };
-  const int pstart = ctop / nb;
-  for (int e = threadIdx.x; STAGE && e < (pstart + 1) * nb * nb; e += blockDim.x) {   // T of panels 0 .. pstart
-    const unsigned sa = static_cast<unsigned>(__cvta_generic_to_shared(Ts + e));
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(T + e));
-  }
-  stage(pstart, 0);   // the same commit group as T
-  for (int pi = pstart; pi >= 0; --pi) {
-    const int k = pstart - pi;
-    if (pi > 0) {
-      stage(pi - 1, (k + 1) & 1);
-      if constexpr (STAGE) asm volatile("cp.async.wait_group 1;\n" ::);
-    } else {
-      if constexpr (STAGE) asm volatile("cp.async.wait_group 0;\n" ::);
-    }
-    __syncthreads();
-    const int p0 = pi * nb, pw = min(nb, n - p0);
-    if (c < n && p0 <= c) {   // warp-uniform
-      const int qb = p0 >> 5, base = p0 & 31, ii = lane - base;   // the panel's rows sit in lanes base ..
-      cd yb = cmk(0.0, 0.0);
-#pragma unroll
-      for (int q = 0; q < QMAX; ++q)
-        if (q == qb) yb = y[q];
-      const cd* Tp = STAGE ? Ts + pi * nb * nb : T + (int64_t)pi * nb * nb;
-      cd a0 = cmk(0.0, 0.0), a1 = cmk(0.0, 0.0);
-      for (int jj = 0; jj < pw; ++jj) {
-        const cd rj = cmk(__shfl_sync(0xffffffffu, yb.x, base + jj), __shfl_sync(0xffffffffu, yb.y, base + jj));
-        if (ii >= 0 && ii <= jj) cfma((jj & 1) ? a1 : a0, Tp[ii + nb * jj], rj);
-      }
-      const cd mi = cadd(a0, a1);
-      if (ii >= 0 && ii < pw) M[p0 + ii + (int64_t)c * n] = mi;
-      const cd* Gc = Gs + (k & 1) * nb * n;
-      for (int jj = 0; jj < pw; ++jj) {
-        const cd mj = cmk(__shfl_sync(0xffffffffu, mi.x, base + jj), __shfl_sync(0xffffffffu, mi.y, base + jj));
-        const cd* gcol = STAGE ? Gc + jj * n : G + (int64_t)(p0 + jj) * n;
-#pragma unroll
-        for (int q = 0; q < QMAX; ++q) {
-          const int r = lane + 32 * q;
-          if (r < p0) y[q] = csub(y[q], cmul(gcol[r], mj));
-        }
-      }
-    }
-    __syncthreads();   // this buffer is refilled by the next iteration's prefetch
-  }
-}
-
-typedef void (*TmatKernel)(int, int, int, const cd*, const cd*, const cd*, cd*);
-
-size_t tmat_smem(int n, int nb) { return (2 * (size_t)nb * n + (size_t)((n + nb - 1) / nb) * nb * nb) * sizeof(cd); }
-
-// The staged variant when G's panel columns (double-buffered) and every T_p fit in shared
-// memory, else the same algorithm reading them from global memory (L2).
-template <bool ST>
-TmatKernel tmat_pick(int n) {
-  if (n <= 32) return qr_tmat_kernel<1, ST>;
-  if (n <= 64) return qr_tmat_kernel<2, ST>;
-  if (n <= 128) return qr_tmat_kernel<4, ST>;
-  if (n <= 256) return qr_tmat_kernel<8, ST>;
-  if (n <= 512) return qr_tmat_kernel<16, ST>;
-  return nullptr;
-}
-TmatKernel tmat_kernel_for(int n, int nb) {
-  return tmat_smem(n, nb) <= SMEM_LIMIT ? tmat_pick<true>(n) : tmat_pick<false>(n);
-}
-
 struct Choice {
-  int C = 0, rpl = 0, nb = 0;
+  int C = 0, rpl = 0, nc = 0;
   size_t smem = 0;
 };
 
-// Cluster of C = ceil(m / (32 rpl)) CTAs, at most 16: prefer 1 row per lane (measured: the
-// per-CTA work, not the exchange, sets the time), then 2, then 4; the widest panel that fits.
-bool choose(int m, int n, Choice& ch) {
+// Cluster of C = ceil(m / (32 rpl)) CTAs, at most 16: prefer 1 row per lane, then 2, then 4; the
+// widest column chunk of the block reflectors that fits.  An outer panel of the blocked form
+// (panel) keeps the columns beside an inner panel in one chunk, since its T needs them.
+bool choose(int m, int n, Choice& ch, bool panel = false) {
   QrParams P;
+  const int nc_max = panel ? std::max(8, (n - NB + 7) / 8 * 8) : std::min(256, (n + 7) / 8 * 8);
+  const int nc_min = panel ? nc_max : 8;
   for (int rpl : {1, 2, 4}) {
     const int rows = 32 * rpl;
     const int C = (m + rows - 1) / rows;
     if (C > CMAX) continue;
-    for (int nb : {16, 8, 4}) {
-      size_t b = layout(P, n, C, rows, nb);
+    for (int nc = nc_max; nc >= nc_min; nc = nc > 16 ? nc / 16 * 8 : nc - 8) {
+      const size_t b = layout(P, n, C, rows, nc);
       if (b <= SMEM_LIMIT) {
-        ch.C = C; ch.rpl = rpl; ch.nb = nb; ch.smem = b;
+        ch.C = C; ch.rpl = rpl; ch.nc = nc; ch.smem = b;
         return true;
       }
     }
@@ -748,44 +882,43 @@ bool choose(int m, int n, Choice& ch) {
   return false;
 }
 
-// Strided m x n matrix fill: COPY dst = src, UPPER dst = triu(src), IDENT dst = [I; 0].
-enum { MAT_COPY = 0, MAT_UPPER, MAT_IDENT };
-__global__ void mat_kernel(int mode, int m, int n, const cd* __restrict__ src, int64_t sr, int64_t sc, cd* dst,
-                           int64_t dr, int64_t dc) {
+// Strided m x n matrix fill for every problem of a batch: COPY dst = src, UPPER dst = triu(src),
+// IDENT dst = [I; 0], CTRANS_UPPER dst = triu(src^H).
+enum { MAT_COPY = 0, MAT_UPPER, MAT_IDENT, MAT_CTRANS_UPPER };
+__global__ void mat_kernel(int mode, int m, int n, const cd* __restrict__ src, int64_t sr, int64_t sc, int64_t sb, cd* dst,
+                           int64_t dr, int64_t dc, int64_t db) {
   const int64_t total = (int64_t)m * n;
+  src += blockIdx.y * sb;
+  dst += blockIdx.y * db;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     const int g = (int)(e % m), k = (int)(e / m);
     cd v;
     if (mode == MAT_IDENT) v = cmk(g == k ? 1.0 : 0.0, 0.0);
-    else if (mode == MAT_UPPER && k < g) v = cmk(0.0, 0.0);
+    else if (mode >= MAT_UPPER && k < g) v = cmk(0.0, 0.0);
+    else if (mode == MAT_CTRANS_UPPER) v = cconj(src[k * sr + g * sc]);
     else v = src[g * sr + k * sc];
     dst[g * dr + k * dc] = v;
   }
 }
 
-int mat_launch(int mode, int m, int n, const cd* src, int64_t sr, int64_t sc, cd* dst, int64_t dr, int64_t dc,
-               Workspace* ws, cudaStream_t s) {
+int mat_launch(int mode, int m, int n, int batch, const cd* src, int64_t sr, int64_t sc, int64_t sb, cd* dst, int64_t dr,
+               int64_t dc, int64_t db, Workspace* ws, cudaStream_t s) {
   count_launch(ws);
   const int64_t total = (int64_t)m * n;
   const int blocks = (int)std::min<int64_t>((total + 255) / 256, 148 * 8);
-  mat_kernel<<<blocks, 256, 0, s>>>(mode, m, n, src, sr, sc, dst, dr, dc);
+  mat_kernel<<<dim3(blocks, batch), 256, 0, s>>>(mode, m, n, src, sr, sc, sb, dst, dr, dc, db);
   MPSB_CUDA_TRY(cudaGetLastError());
   return MPSB_OK;
 }
 
-// The cluster factorisation of every problem of p: R (if requested), the explicit reflectors
-// V [batch][n][m], the panels' T [batch][npanels][nb][nb], and E = [I; 0] in p.Q.
-int launch_factor(const QrProblem& p, const Choice& ch, cd* Vb, cd* Tb, cudaStream_t s) {
-  QrParams P;
-  layout(P, p.n, ch.C, 32 * ch.rpl, ch.nb);
-  P.p = p;
-  P.V = Vb;
-  P.Tg = Tb;
-  QrKernel fn = kernel_for(ch.rpl, ch.nb);
+// The cluster kernel on every problem of p.
+int launch_cluster(QrParams& P, const Choice& ch, cudaStream_t s) {
+  layout(P, P.p.n, ch.C, 32 * ch.rpl, ch.nc);
+  QrKernel fn = kernel_for(ch.rpl, ch.C);
   if (!fn) return MPSB_ERR_UNSUPPORTED;
   MPSB_TRY(ensure_kernel_attrs((const void*)fn, (int)SMEM_LIMIT, true));
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(ch.C, p.batch, 1);
+  cfg.gridDim = dim3(ch.C, P.p.batch, 1);
   cfg.blockDim = dim3(NT, 1, 1);
   cfg.dynamicSmemBytes = ch.smem;
   cfg.stream = s;
@@ -800,47 +933,13 @@ int launch_factor(const QrProblem& p, const Choice& ch, cd* Vb, cd* Tb, cudaStre
   return MPSB_OK;
 }
 
-// Q = E - V (T V1^H) for every problem of p, p.Q holding E: G = V^H V, the back substitution
-// for M = T V1^H, and Q -= V M.
-int form_q(const QrProblem& p, int nb, const cd* Vb, const cd* Tb, cd* Gb, cd* Mb, Workspace* ws, cudaStream_t s) {
-  const int m = p.m, n = p.n;
-  const TmatKernel tk = tmat_kernel_for(n, nb);
-  if (!tk) return MPSB_ERR_UNSUPPORTED;
-  const cd one = cmk(1.0, 0.0), zero = cmk(0.0, 0.0), mone = cmk(-1.0, 0.0);
-  {  // G = V^H V
-    Gemm g;
-    g.M = n; g.N = n; g.K = m; g.batch = p.batch;
-    g.A = Vb; g.a_m = m; g.a_k = 1; g.a_b = (int64_t)m * n; g.conjA = true;
-    g.B = Vb; g.b_k = 1; g.b_n = m; g.b_b = (int64_t)m * n;
-    g.C = Gb; g.c_m = 1; g.c_n = n; g.c_b = (int64_t)n * n;
-    g.alpha = one; g.beta = zero;
-    MPSB_TRY(gemm_launch(g, ws, s));
-  }
-  {  // M = T V1^H
-    const size_t smem = tmat_smem(n, nb) <= SMEM_LIMIT ? tmat_smem(n, nb) : 0;
-    if (smem) MPSB_TRY(ensure_kernel_attrs((const void*)tk, (int)SMEM_LIMIT));
-    count_launch(ws);
-    tk<<<dim3((n + TR_WARPS - 1) / TR_WARPS, p.batch), 32 * TR_WARPS, smem, s>>>(m, n, nb, Vb, Tb, Gb, Mb);
-    MPSB_CUDA_TRY(cudaGetLastError());
-  }
-  {  // Q = E - V M
-    Gemm g;
-    g.M = m; g.N = n; g.K = n; g.batch = p.batch;
-    g.A = Vb; g.a_m = 1; g.a_k = m; g.a_b = (int64_t)m * n;
-    g.B = Mb; g.b_k = 1; g.b_n = n; g.b_b = (int64_t)n * n;
-    g.C = p.Q; g.c_m = p.q_r; g.c_n = p.q_c; g.c_b = p.q_b;
-    g.alpha = mone; g.beta = one;
-    MPSB_TRY(gemm_launch(g, ws, s));
-  }
-  return MPSB_OK;
-}
-
-// Blocked QR for one matrix beyond the cluster's shared memory (for example 2048 x 512): the
-// working matrix is p.Q (X copied in unless they coincide); every 16-column panel is
-// factored by the cluster kernel (its R rows written back in place, its reflectors and T
-// kept), the trailing columns get A -= V (T^H (V^H A)) by three tensor-core GEMMs, and Q is
-// formed from all reflectors as in the single-kernel path.
-constexpr int BP = 16;
+// Blocked QR for matrices beyond the cluster's shared memory (for example 2048 x 512): the working
+// matrix is p.Q (X copied in unless they coincide); every outer panel of up to BP columns is
+// factored by the cluster kernel (its R rows written back in place, its reflectors and T kept), the
+// trailing columns get A -= V (T^H (V^H A)) by three tensor-core GEMMs, and Q is formed from all
+// reflectors.  BP = 64: the widest panel whose 2048 rows fit 16 CTAs' shared memory; the GEMMs'
+// K = 64 then reads and writes the trailing columns n/64 times.
+constexpr int BP = 64;
 
 // The look-ahead lane of the blocked QR: created by the first (eager) call of a workspace.
 int qr_side_lane(Workspace* ws) {
@@ -855,22 +954,32 @@ int qr_side_lane(Workspace* ws) {
   return MPSB_OK;
 }
 
-// Right-looking blocked QR with look-ahead for shapes beyond one cluster (e.g. 2048 x 512):
-// panels of BP columns, each factored by the cluster kernel.  Panel pi's block reflector
-// I - V T V^H is applied to the next panel's columns on the main stream, which then factors
-// that panel at once, while the same update of the columns after it runs on the look-ahead
-// lane -- so the latency-bound panel factorisations overlap the trailing GEMMs.  Every column
-// still gets the panels' updates in panel order (the main stream waits for the lane's update
-// of panel pi-1 before it applies panel pi to the next panel), so the result is the
-// unblocked order's.
+// The widest outer panel that fits one cluster at every row count of the factorisation (0: none).
+int panel_width(int m, int n) {
+  for (int w : {BP, 32, 16}) {
+    w = std::min(w, n);
+    bool ok = true;
+    Choice ch;
+    for (int p0 = 0; p0 < n && ok; p0 += w) ok = choose(m - p0, std::min(w, n - p0), ch, true);
+    if (ok) return w;
+  }
+  return 0;
+}
+
+// Right-looking blocked QR with look-ahead: outer panel pi's block reflector I - V T V^H is applied
+// to the next panel's columns on the main stream, which then factors that panel at once, while the
+// same update of the columns after it runs on the look-ahead lane -- so the latency-bound panel
+// factorisations overlap the trailing GEMMs.  Every column still gets the panels' updates in panel
+// order (the main stream waits for the lane's update of panel pi-1 before it applies panel pi to the
+// next panel), so the result is the unblocked order's.
 int qr_blocked(const QrProblem& p, Workspace* ws, cudaStream_t s) {
-  const int m = p.m, n = p.n, npan = (n + BP - 1) / BP;
+  const int m = p.m, n = p.n, B = p.batch, bp = panel_width(m, n), npan = (n + bp - 1) / bp;
   const int64_t qr_ = p.q_r, qc = p.q_c;
-  // scratch: V [n][m], T [npan][16][16], G and M [n][n], panel V and E [16][m], W and W2 [n][16]
-  // (the lane's trailing update), Wn and W2n [16][16] (the next panel's update)
-  const size_t nV = (size_t)m * n, nT = (size_t)npan * BP * BP, nG = (size_t)n * n, nP = (size_t)m * BP,
-               nW = (size_t)n * BP, nWn = (size_t)BP * BP;
-  MPSB_TRY(devbuf_ensure(ws, ws->qr, (nV + nT + 2 * nG + 2 * nP + 2 * nW + 2 * nWn) * sizeof(cd)));
+  // scratch per problem: V [n][m], T [npan][bp][bp], G, M and B [n][n], W and W2 [n][bp] (the
+  // lane's trailing update), Wn and W2n [bp][bp] (the next panel's update)
+  const int64_t nV = (int64_t)m * n, nT = (int64_t)npan * bp * bp, nG = (int64_t)n * n, nW = (int64_t)n * bp,
+                nWn = (int64_t)bp * bp;
+  MPSB_TRY(devbuf_ensure(ws, ws->qr, (size_t)B * (nV + nT + 3 * nG + 2 * nW + 2 * nWn) * sizeof(cd)));
   MPSB_TRY(qr_side_lane(ws));
   Workspace* sw = ws->qr_side_ws;
   sw->capturing = ws->capturing;
@@ -878,81 +987,65 @@ int qr_blocked(const QrProblem& p, Workspace* ws, cudaStream_t s) {
   cudaStream_t ls = ws->qr_side;
   cudaEvent_t ev_v = ws->qr_ev[0], ev_t = ws->qr_ev[1];
   cd* Vb = static_cast<cd*>(ws->qr.p);
-  cd* Tb = Vb + nV;
-  cd* Gb = Tb + nT;
-  cd* Mb = Gb + nG;
-  cd* Vp = Mb + nG;
-  cd* Ep = Vp + nP;
-  cd* Wb = Ep + nP;
-  cd* W2 = Wb + nW;
-  cd* Wn = W2 + nW;
-  cd* W2n = Wn + nWn;
+  cd* Tb = Vb + B * nV;
+  cd* Gb = Tb + B * nT;
+  cd* Mb = Gb + B * nG;
+  cd* Bb = Mb + B * nG;
+  cd* Wb = Bb + B * nG;
+  cd* W2 = Wb + B * nW;
+  cd* Wn = W2 + B * nW;
+  cd* W2n = Wn + B * nWn;
   cd* A = p.Q;
-  if (p.X != p.Q || p.x_r != qr_ || p.x_c != qc)
-    MPSB_TRY(mat_launch(MAT_COPY, m, n, p.X, p.x_r, p.x_c, A, qr_, qc, ws, s));
-  MPSB_CUDA_TRY(cudaMemsetAsync(Vb, 0, nV * sizeof(cd), s));
+  if (p.X != p.Q || p.x_r != qr_ || p.x_c != qc || p.x_b != p.q_b)
+    MPSB_TRY(mat_launch(MAT_COPY, m, n, B, p.X, p.x_r, p.x_c, p.x_b, A, qr_, qc, p.q_b, ws, s));
+  MPSB_CUDA_TRY(cudaMemsetAsync(Vb, 0, (size_t)B * nV * sizeof(cd), s));
   const cd one = cmk(1.0, 0.0), zero = cmk(0.0, 0.0), mone = cmk(-1.0, 0.0);
 
-  // factor panel pi (its columns have every earlier panel's update) and keep its V in Vb
+  // factor panel pi (its columns have every earlier panel's update)
   auto factor = [&](int pi) -> int {
-    const int p0 = pi * BP, pw = std::min(BP, n - p0), mp = m - p0;
+    const int p0 = pi * bp, pw = std::min(bp, n - p0), mp = m - p0;
     Choice ch;
-    if (!choose(mp, pw, ch) || ch.nb != BP) {
+    if (!choose(mp, pw, ch, true)) {
       set_last_message("QR panel of %d x %d does not fit the cluster kernel", mp, pw);
       return MPSB_ERR_UNSUPPORTED;
     }
-    cd* Ap = A + p0 * qr_ + p0 * qc;
-    QrProblem pp;
-    pp.m = mp; pp.n = pw; pp.batch = 1;
-    pp.X = Ap; pp.x_r = qr_; pp.x_c = qc;
-    pp.Q = Ep; pp.q_r = 1; pp.q_c = mp;
-    pp.R = Ap; pp.r_r = qr_; pp.r_c = qc;   // R rows back in place (the panel's V is kept apart)
-    pp.err = p.err;
+    QrParams P = {};
+    P.p = p;
+    P.p.m = mp; P.p.n = pw;
+    P.p.X = A + p0 * qr_ + p0 * qc; P.p.x_r = qr_; P.p.x_c = qc; P.p.x_b = p.q_b;
+    P.p.Q = nullptr;
+    P.p.R = A + p0 * qr_ + p0 * qc; P.p.r_r = qr_; P.p.r_c = qc; P.p.r_b = p.q_b;   // R rows back in place
+    P.form_q = 0;
+    P.V = Vb + p0 + (int64_t)p0 * m; P.v_ld = m; P.v_b = nV;
+    P.T = Tb + (int64_t)pi * bp * bp; P.t_ld = bp; P.t_b = nT;
     count_launch(ws);
-    MPSB_TRY(launch_factor(pp, ch, Vp, Tb + (int64_t)pi * BP * BP, s));
-    MPSB_CUDA_TRY(cudaMemcpy2DAsync(Vb + p0 + (int64_t)p0 * m, (size_t)m * sizeof(cd), Vp, (size_t)mp * sizeof(cd),
-                                    (size_t)mp * sizeof(cd), pw, cudaMemcpyDeviceToDevice, s));
-    return MPSB_OK;
+    return launch_cluster(P, ch, s);
+  };
+  auto gemm = [&](int M, int N, int K, const cd* Ap, int64_t am, int64_t ak, int64_t ab, bool ca, const cd* Bp, int64_t bk,
+                  int64_t bn, int64_t bb, cd* Cp, int64_t cm, int64_t cn, int64_t cb, cd alpha, cd beta, Workspace* w,
+                  cudaStream_t st) -> int {
+    Gemm g;
+    g.M = M; g.N = N; g.K = K; g.batch = B;
+    g.A = Ap; g.a_m = am; g.a_k = ak; g.a_b = ab; g.conjA = ca;
+    g.B = Bp; g.b_k = bk; g.b_n = bn; g.b_b = bb;
+    g.C = Cp; g.c_m = cm; g.c_n = cn; g.c_b = cb;
+    g.alpha = alpha; g.beta = beta;
+    return gemm_launch(g, w, st);
   };
   // columns c0 .. c0 + nc - 1 of A <- (I - V T V^H)^H applied by panel pi, on stream st
-  auto update = [&](int pi, int c0, int nc, cd* W, int ldw, cd* Wt, Workspace* w, cudaStream_t st) -> int {
-    const int p0 = pi * BP, pw = std::min(BP, n - p0), mp = m - p0;
+  auto update = [&](int pi, int c0, int nc, cd* W, cd* Wt, int64_t wb, Workspace* w, cudaStream_t st) -> int {
+    const int p0 = pi * bp, pw = std::min(bp, n - p0), mp = m - p0;
     const cd* V = Vb + p0 + (int64_t)p0 * m;   // rows p0.., leading dimension m
     cd* At = A + p0 * qr_ + (int64_t)c0 * qc;
-    {  // W = V^H A_t
-      Gemm g;
-      g.M = pw; g.N = nc; g.K = mp;
-      g.A = V; g.a_m = m; g.a_k = 1; g.conjA = true;
-      g.B = At; g.b_k = qr_; g.b_n = qc;
-      g.C = W; g.c_m = 1; g.c_n = ldw;
-      g.alpha = one; g.beta = zero;
-      MPSB_TRY(gemm_launch(g, w, st));
-    }
-    {  // Wt = T^H W
-      Gemm g;
-      g.M = pw; g.N = nc; g.K = pw;
-      g.A = Tb + (int64_t)pi * BP * BP; g.a_m = BP; g.a_k = 1; g.conjA = true;
-      g.B = W; g.b_k = 1; g.b_n = ldw;
-      g.C = Wt; g.c_m = 1; g.c_n = ldw;
-      g.alpha = one; g.beta = zero;
-      MPSB_TRY(gemm_launch(g, w, st));
-    }
-    {  // A_t -= V Wt
-      Gemm g;
-      g.M = mp; g.N = nc; g.K = pw;
-      g.A = V; g.a_m = 1; g.a_k = m;
-      g.B = Wt; g.b_k = 1; g.b_n = ldw;
-      g.C = At; g.c_m = qr_; g.c_n = qc;
-      g.alpha = mone; g.beta = one;
-      MPSB_TRY(gemm_launch(g, w, st));
-    }
-    return MPSB_OK;
+    MPSB_TRY(gemm(pw, nc, mp, V, m, 1, nV, true, At, qr_, qc, p.q_b, W, 1, bp, wb, one, zero, w, st));    // V^H A
+    MPSB_TRY(gemm(pw, nc, pw, Tb + (int64_t)pi * bp * bp, bp, 1, nT, true, W, 1, bp, wb, Wt, 1, bp, wb, one, zero, w, st));
+    return gemm(mp, nc, pw, V, 1, m, nV, false, Wt, 1, bp, wb, At, qr_, qc, p.q_b, mone, one, w, st);     // A -= V Wt
   };
 
   MPSB_TRY(factor(0));
   bool lane_pending = false;   // the lane holds an update the main stream has not waited for
   for (int pi = 0; pi + 1 < npan; ++pi) {
-    const int c1 = (pi + 1) * BP, nnext = std::min(BP, n - c1);
+    const int c1 = (pi + 1) * bp, nnext = std::min(bp, n - c1);
     const int c2 = c1 + nnext, nrest = n - c2;
     // the next panel's columns have panel pi-1's update only once the lane's update is done
     if (lane_pending) {
@@ -963,11 +1056,11 @@ int qr_blocked(const QrProblem& p, Workspace* ws, cudaStream_t s) {
     if (nrest > 0) {   // V_pi and T_pi are final on the main stream: fork the trailing update
       MPSB_CUDA_TRY(cudaEventRecord(ev_v, s));
       MPSB_CUDA_TRY(cudaStreamWaitEvent(ls, ev_v, 0));
-      st = update(pi, c2, nrest, Wb, BP, W2, sw, ls);
+      st = update(pi, c2, nrest, Wb, W2, nW, sw, ls);
       MPSB_CUDA_TRY(cudaEventRecord(ev_t, ls));   // recorded on failure too, so the join below holds
       lane_pending = true;
     }
-    if (st == MPSB_OK) st = update(pi, c1, nnext, Wn, BP, W2n, ws, s);
+    if (st == MPSB_OK) st = update(pi, c1, nnext, Wn, W2n, nWn, ws, s);
     if (st == MPSB_OK) st = factor(pi + 1);
     if (st != MPSB_OK) {   // never leave the lane forked
       cudaStreamWaitEvent(s, ev_t, 0);
@@ -977,27 +1070,32 @@ int qr_blocked(const QrProblem& p, Workspace* ws, cudaStream_t s) {
   if (lane_pending) MPSB_CUDA_TRY(cudaStreamWaitEvent(s, ev_t, 0));   // join the lane
   ws->launches += sw->launches;
   sw->launches = 0;
-  if (p.R) MPSB_TRY(mat_launch(MAT_UPPER, n, n, A, qr_, qc, p.R, p.r_r, p.r_c, ws, s));
-  MPSB_TRY(mat_launch(MAT_IDENT, m, n, nullptr, 0, 0, A, qr_, qc, ws, s));
-  QrProblem q = p;
-  return form_q(q, BP, Vb, Tb, Gb, Mb, ws, s);
-}
+  if (p.R) MPSB_TRY(mat_launch(MAT_UPPER, n, n, B, A, qr_, qc, p.q_b, p.R, p.r_r, p.r_c, p.r_b, ws, s));
+  MPSB_TRY(mat_launch(MAT_IDENT, m, n, B, A, 0, 0, 0, A, qr_, qc, p.q_b, ws, s));
 
-bool blocked_ok(int m, int n) {
-  Choice ch;
-  return n <= 512 && choose(m, std::min(n, BP), ch) && ch.nb == BP;
+  // Q = E - V M, M = T V1^H by back substitution over the outer panels: T^{-1} = diag(1/tau) +
+  // striu(V^H V) is block upper triangular with the panels' T_p inverted on its diagonal, so with
+  // G = V^H V and B = V1^H (upper triangular)  M_p = T_p (B_p - sum_{q > p} G_pq M_q), p = last .. 0
+  // (no division; zero rows for tau = 0 reflectors).
+  MPSB_TRY(gemm(n, n, m, Vb, m, 1, nV, true, Vb, 1, m, nV, Gb, 1, n, nG, one, zero, ws, s));
+  MPSB_TRY(mat_launch(MAT_CTRANS_UPPER, n, n, B, Vb, 1, m, nV, Bb, 1, n, nG, ws, s));
+  MPSB_CUDA_TRY(cudaMemsetAsync(Mb, 0, (size_t)B * nG * sizeof(cd), s));
+  for (int pi = npan - 1; pi >= 0; --pi) {
+    const int p0 = pi * bp, pw = std::min(bp, n - p0), kb = p0 + pw, nt = n - kb;
+    if (nt > 0)
+      MPSB_TRY(gemm(pw, nt, nt, Gb + p0 + (int64_t)kb * n, 1, n, nG, false, Mb + kb + (int64_t)kb * n, 1, n, nG,
+                    Bb + p0 + (int64_t)kb * n, 1, n, nG, mone, one, ws, s));
+    MPSB_TRY(gemm(pw, pw + nt, pw, Tb + (int64_t)pi * bp * bp, 1, bp, nT, false, Bb + p0 + (int64_t)p0 * n, 1, n, nG,
+                  Mb + p0 + (int64_t)p0 * n, 1, n, nG, one, zero, ws, s));
+  }
+  return gemm(m, n, n, Vb, 1, m, nV, false, Mb, 1, n, nG, A, qr_, qc, p.q_b, mone, one, ws, s);
 }
 
 }  // namespace
 
-bool qr_batch_supported(int m, int n) {
-  Choice ch;
-  return m >= n && n >= 1 && n <= 512 && choose(m, n, ch);
-}
-
 bool qr_supported(int m, int n) {
   Choice ch;
-  return m >= n && n >= 1 && n <= 512 && (choose(m, n, ch) || blocked_ok(m, n));
+  return m >= n && n >= 1 && n <= 512 && (choose(m, n, ch) || panel_width(m, n) > 0);
 }
 
 int qr_launch(const QrProblem& p, Workspace* ws, cudaStream_t s) {
@@ -1005,23 +1103,20 @@ int qr_launch(const QrProblem& p, Workspace* ws, cudaStream_t s) {
   if (p.batch > 65535) return MPSB_ERR_UNSUPPORTED;
   if (!ws) return MPSB_ERR_INVALID_ARG;
   const int m = p.m, n = p.n;
-  Choice ch;
-  if (n > 512 || (!choose(m, n, ch) && (p.batch != 1 || !blocked_ok(m, n)))) {
+  if (!qr_supported(m, n)) {
     set_last_message("QR of a %d x %d matrix (batch %d) is beyond the supported shapes", m, n, p.batch);
     return MPSB_ERR_UNSUPPORTED;
   }
+  Choice ch;
   if (!choose(m, n, ch)) return qr_blocked(p, ws, s);
-  const int nb = ch.nb, npan = (n + nb - 1) / nb;
-  // scratch: V [batch][n][m], the panels' T [batch][npan][nb][nb], G = V^H V and
-  // M = T V1^H [batch][n][n] each
-  const size_t nV = (size_t)p.batch * m * n, nT = (size_t)p.batch * npan * nb * nb, nG = (size_t)p.batch * n * n;
-  MPSB_TRY(devbuf_ensure(ws, ws->qr, (nV + nT + 2 * nG) * sizeof(cd)));
-  cd* Vb = static_cast<cd*>(ws->qr.p);
-  cd* Tb = Vb + nV;
-  cd* Gb = Tb + nT;
-  cd* Mb = Gb + nG;
-  MPSB_TRY(launch_factor(p, ch, Vb, Tb, s));
-  return form_q(p, nb, Vb, Tb, Gb, Mb, ws, s);
+  const int64_t nT = (int64_t)((n + NB - 1) / NB) * NB * NB;
+  MPSB_TRY(devbuf_ensure(ws, ws->qr, (size_t)p.batch * nT * sizeof(cd)));
+  QrParams P = {};
+  P.p = p;
+  P.form_q = 1;
+  P.T = static_cast<cd*>(ws->qr.p);
+  P.t_b = nT;
+  return launch_cluster(P, ch, s);
 }
 
 }  // namespace mpsb

@@ -15,7 +15,7 @@ struct DevBuf {
 
 struct Workspace {
   DevBuf splitk;          // split-K partial tiles
-  DevBuf qr;              // QR: reflectors, tau, V^H V and T V1^H
+  DevBuf qr;              // QR: the panels' T; blocked form also reflectors, V^H V and T V1^H
   DevBuf svd;             // SVD: the Jacobi working matrix, V, norms, flags
   DevBuf oz;              // sliced tensor-core GEMM: int8 slices of both operands, row exponents
   DevBuf named[16];       // per-sweep temporaries (see engine.cu)
