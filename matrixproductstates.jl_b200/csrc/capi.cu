@@ -44,7 +44,7 @@ static int sync(mpsb_ctx* ctx) {
     cudaMemsetAsync(ctx->err(), 0, sizeof(int), ctx->stream);
     cudaStreamSynchronize(ctx->stream);
     set_last_message("a device-side wait timed out (%s); results of this stream are invalid",
-                     (word & 4) ? "wait self-test" : (word & 2) ? "sliced GEMM pipeline" : "QR cluster exchange");
+                     (word & 4) ? "wait self-test" : (word & 2) ? "sliced GEMM pipeline" : (word & 8) ? "GEMM pipeline" : "QR cluster exchange");
     return MPSB_ERR_CUDA;
   }
   return MPSB_OK;
@@ -151,6 +151,7 @@ int mpsb_ctx_create(int device, mpsb_ctx** out) {
     set_last_message("allocation of context scalars failed");
     return MPSB_ERR_OUT_OF_MEMORY;
   }
+  c->ws.err = c->ws_side.err = c->err();
   cudaMemset(c->d_scalars, 0, 64 * sizeof(double));
   c->h_scalars[63] = 0.0;
   *out = c;

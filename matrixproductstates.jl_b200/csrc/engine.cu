@@ -101,10 +101,7 @@ int run_gemm(mpsb_ctx* ctx, const Gemm& g0) {
     if (ctx->ws.oz.p != before_oz) ctx->ws_generation++;
     return ozgemm_launch(g, ctx->split_slices, ctx->ws.oz.p, ctx->ws.oz.cap, ctx->err(), &ctx->ws, ctx->stream);
   }
-  void* before = ctx->ws.splitk.p;
-  int st = gemm_launch(g, &ctx->ws, ctx->stream);
-  if (ctx->ws.splitk.p != before) ctx->ws_generation++;
-  return st;
+  return gemm_launch(g, &ctx->ws, ctx->stream);
 }
 
 static inline int run_mpo(mpsb_ctx* ctx, const MpoApply& a0, int64_t k1, int64_t k2, int64_t m1, int64_t m2) {
@@ -250,8 +247,7 @@ int op_update_lenv(mpsb_ctx* ctx, const cd* A0, const cd* AL, cd* env, int lead,
   return run_gemm(ctx, g);
 }
 
-// QR through the context's workspace; a reallocated QR or split-K scratch (the blocked QR's
-// trailing GEMMs may split K) invalidates captured graphs
+// QR through the context's workspace; a reallocated QR scratch invalidates captured graphs
 int run_qr(mpsb_ctx* ctx, const QrProblem& p0) {
   QrProblem p = p0;
   if (ctx->batch > 1 && p.batch == 1) {
@@ -261,12 +257,9 @@ int run_qr(mpsb_ctx* ctx, const QrProblem& p0) {
     p.batch = ctx->batch;
   }
   void* before = ctx->ws.qr.p;
-  void* before_sk = ctx->ws.splitk.p;
-  void* before_side = ctx->ws.qr_side_ws ? ctx->ws.qr_side_ws->splitk.p : nullptr;
   count_launch(&ctx->ws);
   const int st = qr_launch(p, &ctx->ws, ctx->stream);
-  void* after_side = ctx->ws.qr_side_ws ? ctx->ws.qr_side_ws->splitk.p : nullptr;
-  if (ctx->ws.qr.p != before || ctx->ws.splitk.p != before_sk || after_side != before_side) ctx->ws_generation++;
+  if (ctx->ws.qr.p != before) ctx->ws_generation++;
   return st;
 }
 

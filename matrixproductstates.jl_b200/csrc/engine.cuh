@@ -49,7 +49,7 @@ struct mpsb_ctx {
   double* d_scalars = nullptr; // small device scratch for norms (64 doubles)
   double* h_scalars = nullptr; // pinned host mirror
   // device error word (inside d_scalars[63]): kernels whose bounded waits run out set a bit
-  // (bit 0: the QR cluster's exchanges, bit 1: the sliced GEMM's pipeline)
+  // (bit 0: the QR cluster's exchanges, bit 1: the sliced GEMM's pipeline, bit 3: the FP64 GEMM's)
   int* err() const { return reinterpret_cast<int*>(d_scalars + 63); }
   struct GraphEntry {
     cudaGraphExec_t exec = nullptr;

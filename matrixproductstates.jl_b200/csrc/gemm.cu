@@ -5,211 +5,308 @@
 // (m, k[, batch]) element-stride triple, so reference transposes ('), (.') and the
 // reshape/permutedims chains cost no copies.
 //
-// Tiling (FP64 tensor path, DMMA): 64x64 complex C tile per 128-thread CTA; each warp owns
-// 32x32 complex as 2x4 blocks of 16x8 and issues mma.sync.m16n8k8.f64 -- four real products
-// per complex k8 step (Re += Ar Br - Ai Bi, Im += Ar Bi + Ai Br) -- with every fragment
-// element loaded as one 16-byte (re, im) pair from shared memory.  K is staged 16 complex
-// deep through a three-stage cp.async ring (3 x 2 x 16 x 66 x 16 B = 101 KB, two CTAs per
-// SM); the row pitch of 66 elements puts the eight 16-byte fragment loads of a quarter warp
-// in eight distinct bank groups.  Skinny problems split K across CTAs into a workspace that a
-// second kernel sums in a fixed order, so results are bitwise reproducible run to run.
+// Tiling (FP64 tensor path, DMMA): a 32 x 32 complex C tile per 256-thread CTA, as blocks of 16x8 by
+// mma.sync.m16n8k8.f64 -- four real products per complex k8 step (Re += Ar Br - Ai Bi,
+// Im += Ar Bi + Ai Br) -- with every fragment element loaded as one 16-byte (re, im) pair from
+// shared memory.  Two groups of 2 x 2 warps take one k8 step each of every 16-deep stage (so a CTA
+// alone on its SM still has two warps per scheduler to hide the fragment loads) and their partial
+// tiles are added at the end.  Stages come through a four-deep ring of tiled TMA copies (mbarrier
+// byte counts, zero fill outside the matrix) into 128-byte rows of eight elements, 128-byte swizzle;
+// a quarter warp's eight 16-byte fragment loads then fall into eight distinct bank groups, for
+// either contiguous index.  Problems with few tiles also split K over the CTAs of a thread-block
+// cluster, which sum their partial tiles over distributed shared memory.  All sums run in a fixed
+// order, so results are bitwise reproducible run to run, and no partial goes through global memory.
+//
+// What bounds it: the FP64 tensor pipe (64 FMA a clock and SM) on large problems, 33 of 36.8 TFLOP/s;
+// a stage's latency (1475 clocks against 1024 of tensor work) where a CTA has its SM alone.  Tiles of
+// 64 x 64 were slower at every size measured (fewer CTAs to overlap, and one tile of K = 64 is 8.5 us
+// of one SM); copies by the threads' cp.async ran at 12-18 B a clock and SM, 1.3-2 us a stage.
+// Against that form with 64 x 64 tiles and split-K partials through global memory (B200): 512 x 2048 x
+// 4096 (A along K) 1439 -> 1030 us, 2048 x 512 x 512 178 -> 139, 512 x 512 x 2048 227 -> 156, 128 x 512 x
+// 1024 36.6 -> 26.7.
+#include <cooperative_groups.h>
+
+#include <algorithm>
+#include <cmath>
+
 #include "common.cuh"
+#include "tma.cuh"
 #include "workspace.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace mpsb {
 
 namespace {
 
-constexpr int BM = 64, BN = 64, BK = 16, NT = 128, PAD = 2, STAGES = 3;
-constexpr int LDA_S = BM + PAD, LDB_S = BN + PAD;
-constexpr size_t STAGE_ELEMS = size_t(BK) * LDA_S + size_t(BK) * LDB_S;
-constexpr size_t SMEM_BYTES = STAGES * STAGE_ELEMS * sizeof(cd);
+constexpr int T = 32, BK = 16, NT = 256, STAGES = 4, SPLIT_MAX = 16;
+constexpr int LDS = T + 2, LDP = T + 1;              // row pitch of a copied stage, column pitch of a partial tile
+constexpr int OPERAND = T * BK;                      // elements of one operand's TMA stage
+constexpr int STAGE = 2 * BK * LDS;                  // elements of a copied stage (A then B)
+constexpr int PART = T * LDP;                        // elements of a partial tile
+constexpr int CP_STAGES = 3;
+constexpr size_t SMEM_TMA = (size_t)STAGES * 2 * OPERAND * sizeof(cd) + 1024 + STAGES * sizeof(uint64_t);
+constexpr size_t SMEM_COPY = (size_t)CP_STAGES * STAGE * sizeof(cd);
+constexpr int WAIT_LIMIT = 1 << 20;
+static_assert(2 * PART <= CP_STAGES * STAGE && 2 * PART <= STAGES * 2 * OPERAND, "the partial tiles reuse the stages");
 
 struct GemmParams {
   Gemm g;
-  int splits;
-  int kt_per_split;   // K tiles per split
-  cd* ws;             // [split][batch][N][M] partials when splits > 1
+  int kt_per_split;   // stages per split (cluster dimension y = the splits)
+  int* err;           // device error word (may be null)
 };
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool pred) {
-  unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-  int sz = pred ? 16 : 0;
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(sz));
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
-
-template <bool A_MCONTIG, bool B_KCONTIG>
-__device__ __forceinline__ void load_tile(cd* As, cd* Bs, const cd* A, const cd* B, const Gemm& g,
-                                          int m0, int n0, int k0, int tid) {
-  // A tile: BM x BK, stored As[k][m]
+// The sum of the groups' (and, over the cluster, the splits') partial tiles, C = alpha sum + beta C.
+// Accumulator (j, e): row wm + 8(e/2) + fg, column wn + 8j + 2ft + e%2 of the group's partial tile.
+__device__ __forceinline__ void finish_tile(const GemmParams& P, cd* smem, const double (&cr)[2][4], const double (&ci)[2][4],
+                                            int m0, int n0) {
+  const Gemm& g = P.g;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, split = blockIdx.y, splits = gridDim.y;
+  const int wm = (warp & 1) * 16, wn = ((warp >> 1) & 1) * 16, fg = lane >> 2, ft = lane & 3;
+  cd* part = smem + (warp >> 2) * PART;
 #pragma unroll
-  for (int i = 0; i < (BM * BK) / NT; ++i) {
-    int m, k;
-    if (A_MCONTIG) { m = tid % BM; k = tid / BM + (NT / BM) * i; }
-    else           { k = tid % BK; m = tid / BK + (NT / BK) * i; }
-    int gm = m0 + m, gk = k0 + k;
-    bool ok = (gm < g.M) && (gk < g.K);
-    const cd* src = ok ? (A + (int64_t)gm * g.a_m + (int64_t)gk * g.a_k) : A;
-    cp_async16(As + k * LDA_S + m, src, ok);
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      part[(wn + 8 * j + 2 * ft + (e & 1)) * LDP + wm + 8 * (e >> 1) + fg] = cmk(cr[j][e], ci[j][e]);
+  cg::cluster_group cluster = cg::this_cluster();
+  if (splits > 1) cluster.sync();
+  else __syncthreads();
+  // rank r sums columns r, r + splits, ... of the tile over the ranks' groups in order
+  cd* C = g.C + (int64_t)blockIdx.z * g.c_b;
+  const bool use_beta = (g.beta.x != 0.0) || (g.beta.y != 0.0);
+  const int m = tid % T;
+  if (m0 + m < g.M) {
+    for (int n = split + splits * (tid / T); n < T && n0 + n < g.N; n += splits * (NT / T)) {
+      cd* src = &smem[n * LDP + m];
+      cd v;
+      if (splits > 1) {
+        v = cmk(0.0, 0.0);
+#pragma unroll 4
+        for (int q = 0; q < splits; ++q) {
+          const cd* rs = cluster.map_shared_rank(src, q);
+          v = cadd(v, cadd(rs[0], rs[PART]));
+        }
+      } else {
+        v = cadd(src[0], src[PART]);
+      }
+      cd* c = C + (int64_t)(m0 + m) * g.c_m + (int64_t)(n0 + n) * g.c_n;
+      v = cmul(g.alpha, v);
+      if (use_beta) v = cadd(v, cmul(g.beta, *c));
+      *c = v;
+    }
   }
-  // B tile: BK x BN, stored Bs[k][n]
+  if (splits > 1) cluster.sync();   // no CTA leaves while a peer reads its partials
+}
+
+// One complex k8 step of a warp's 16 x 16 block.  Re += Ar Br - Ai Bi, Im += Ar Bi + Ai Br, term-major
+// so one accumulator's two products sit four issues apart.
+__device__ __forceinline__ void mma_k8(double (&cr)[2][4], double (&ci)[2][4], const cd (&a)[4], const cd (&b)[2][2],
+                                       bool conjA, bool conjB) {
+  double ar[4], ai[4], nai[4], br[2][2], bi[2][2];
 #pragma unroll
-  for (int i = 0; i < (BN * BK) / NT; ++i) {
-    int n, k;
-    if (B_KCONTIG) { k = tid % BK; n = tid / BK + (NT / BK) * i; }
-    else           { n = tid % BN; k = tid / BN + (NT / BN) * i; }
-    int gn = n0 + n, gk = k0 + k;
-    bool ok = (gn < g.N) && (gk < g.K);
-    const cd* src = ok ? (B + (int64_t)gk * g.b_k + (int64_t)gn * g.b_n) : B;
-    cp_async16(Bs + k * LDB_S + n, src, ok);
+  for (int e = 0; e < 4; ++e) {
+    ar[e] = a[e].x;
+    ai[e] = conjA ? -a[e].y : a[e].y;
+    nai[e] = -ai[e];
+  }
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      br[j][e] = b[j][e].x;
+      bi[j][e] = conjB ? -b[j][e].y : b[j][e].y;
+    }
+#pragma unroll
+  for (int j = 0; j < 2; ++j) dmma16(cr[j], ar, br[j]);
+#pragma unroll
+  for (int j = 0; j < 2; ++j) dmma16(ci[j], ar, bi[j]);
+#pragma unroll
+  for (int j = 0; j < 2; ++j) dmma16(cr[j], nai, bi[j]);
+#pragma unroll
+  for (int j = 0; j < 2; ++j) dmma16(ci[j], ai, br[j]);
+}
+
+__device__ __forceinline__ uint32_t su32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
+__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {   // bounded
+  for (int it = 0; it < WAIT_LIMIT; ++it) {
+    uint32_t ok;
+    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+
+// An operand's 32 x 16 stage: free index contiguous -- four boxes of 8 (free) x 16 (k), box g at g * 2 KB,
+// a row per k; k contiguous -- two boxes of 8 (k) x 32 (free), box h at h * 4 KB, a row per free
+// index.  Chunk c of row r sits at c ^ (r mod 8).
+template <bool FREE_CONTIG>
+__device__ __forceinline__ void tma_stage(uint32_t dst, const CUtensorMap* map, uint32_t bar, int f0, int k0, int b) {
+#pragma unroll
+  for (int q = 0; q < (FREE_CONTIG ? 4 : 2); ++q) {
+    const int x = 2 * (FREE_CONTIG ? f0 + 8 * q : k0 + 8 * q), y = FREE_CONTIG ? k0 : f0;
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n" ::
+                     "r"(dst + q * (FREE_CONTIG ? 2048 : 4096)), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y),
+                 "r"(b) : "memory");
   }
 }
 
 template <bool CONJA, bool CONJB, bool A_MCONTIG, bool B_KCONTIG>
-__global__ void __launch_bounds__(NT, 2) zgemm_kernel(GemmParams P) {
+__global__ void __launch_bounds__(NT, 3) zgemm_tma_kernel(const __grid_constant__ CUtensorMap ma,
+                                                          const __grid_constant__ CUtensorMap mb, GemmParams P) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  constexpr uint32_t OP_BYTES = OPERAND * sizeof(cd);
+  const Gemm& g = P.g;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tiles_m = (g.M + T - 1) / T;
+  const int m0 = (blockIdx.x % tiles_m) * T, n0 = (blockIdx.x / tiles_m) * T;
+  const int KT = (g.K + BK - 1) / BK, kt0 = blockIdx.y * P.kt_per_split;
+  const int nkt = max(0, min(KT, kt0 + P.kt_per_split) - kt0);
+  const int ba = g.a_b ? blockIdx.z : 0, bb = g.b_b ? blockIdx.z : 0;
+  const uint32_t ring32 = su32(ring), bars = ring32 + STAGES * 2 * OP_BYTES;
+
+  auto issue = [&](int t) {   // thread 0: stage t into its slot
+    const uint32_t bar = bars + 8 * (t % STAGES), dst = ring32 + (t % STAGES) * 2 * OP_BYTES;
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(2 * OP_BYTES) : "memory");
+    tma_stage<A_MCONTIG>(dst, &ma, bar, m0, (kt0 + t) * BK, ba);
+    tma_stage<!B_KCONTIG>(dst + OP_BYTES, &mb, bar, n0, (kt0 + t) * BK, bb);
+  };
+  if (tid == 0) {
+    for (int i = 0; i < STAGES; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bars + 8 * i) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    for (int t = 0; t < STAGES - 1 && t < nkt; ++t) issue(t);
+  }
+  __syncthreads();
+
+  // this warp's fragments: k index t <-> row 2 t of its half stage, t + 4 <-> 2 t + 1
+  const int grp = warp >> 2, wm = (warp & 1) * 16, wn = ((warp >> 1) & 1) * 16, fg = lane >> 2, ft = lane & 3;
+  uint32_t oa[2], ob[2];   // of k rows 2 ft and 2 ft + 1
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const uint32_t k = 8 * grp + 2 * ft + h, c = (uint32_t)((2 * ft + h) ^ fg) << 4;
+    oa[h] = c + (A_MCONTIG ? (wm >> 3) * 2048 + k * 128 : grp * 4096 + (wm + fg) * 128);
+    ob[h] = c + (!B_KCONTIG ? (wn >> 3) * 2048 + k * 128 : grp * 4096 + (wn + fg) * 128);
+  }
+  constexpr uint32_t FA = A_MCONTIG ? 2048 : 8 * 128, FB = !B_KCONTIG ? 2048 : 8 * 128;   // 8 free indices on
+  double cr[2][4], ci[2][4];
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) cr[j][e] = ci[j][e] = 0.0;
+  bool failed = false;
+#pragma unroll 1
+  for (int t = 0; t < nkt; ++t) {
+    if (!failed && !bar_wait(bars + 8 * (t % STAGES), (uint32_t)(t / STAGES) & 1)) {
+      failed = true;
+      if (P.err) atomicOr(P.err, 8);
+    }
+    __syncthreads();   // every warp is done with the slot of stage t - 1
+    if (tid == 0 && t + STAGES - 1 < nkt && !failed) issue(t + STAGES - 1);
+    const unsigned char* sa = ring + (t % STAGES) * 2 * OP_BYTES;
+    const unsigned char* sb = sa + OP_BYTES;
+    cd a[4], b[2][2];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) a[e] = *reinterpret_cast<const cd*>(sa + oa[e >> 1] + (e & 1) * FA);
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) b[j][e] = *reinterpret_cast<const cd*>(sb + ob[e] + j * FB);
+    mma_k8(cr, ci, a, b, CONJA, CONJB);
+  }
+  if (failed && tid == 0) {   // the copies in flight land (or the bound ends) before the CTA goes away
+    for (int t = max(0, nkt - STAGES); t < nkt; ++t) bar_wait(bars + 8 * (t % STAGES), (uint32_t)(t / STAGES) & 1);
+  }
+  __syncthreads();   // every warp is done with the stages
+  finish_tile(P, reinterpret_cast<cd*>(ring), cr, ci, m0, n0);
+}
+
+// The same tile with stages copied by the threads, for operands that a tensor map does not describe
+// (neither index contiguous, or a stride outside its range).
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
+
+// One operand's stages (T x 16, stored [k][free]), zero outside the matrix: this thread's two elements
+// of a stage are p and p + di, and p moves by dk per stage.
+struct Stream {
+  const cd* base;
+  const cd* p;
+  int64_t di, dk;
+  unsigned dst;   // byte offset in the stage
+  int k;          // this thread's k in a stage
+  bool in;        // its free index is inside
+  __device__ Stream(const cd* b, int64_t s_free, int64_t s_k, int f0, int extent, int k0, int tid) : base(b) {
+    const int f = tid % T;
+    k = tid / T;
+    p = b + (int64_t)(f0 + f) * s_free + (int64_t)(k0 + k) * s_k;
+    di = (NT / T) * s_k;
+    dk = BK * s_k;
+    dst = (unsigned)((k * LDS + f) * sizeof(cd));
+    in = f0 + f < extent;
+  }
+  __device__ __forceinline__ void load(unsigned st, int krem) {   // krem: the matrix's k extent from this stage on
+#pragma unroll
+    for (int i = 0; i < T * BK / NT; ++i) {
+      const bool ok = in && k + i * (NT / T) < krem;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(st + dst + i * (unsigned)((NT / T) * LDS * sizeof(cd))),
+                   "l"(ok ? p + i * di : base), "r"(ok ? 16 : 0));
+    }
+    p += dk;
+  }
+};
+
+template <bool CONJA, bool CONJB>
+__global__ void __launch_bounds__(NT, 3) zgemm_copy_kernel(GemmParams P) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cd* smem = reinterpret_cast<cd*>(smem_raw);
   const Gemm& g = P.g;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int tiles_m = (g.M + BM - 1) / BM;
-  const int m0 = (blockIdx.x % tiles_m) * BM;
-  const int n0 = (blockIdx.x / tiles_m) * BN;
-  const int split = blockIdx.y;
-  const int b = blockIdx.z;
-  const cd* A = g.A + (int64_t)b * g.a_b;
-  const cd* B = g.B + (int64_t)b * g.b_b;
+  const int tiles_m = (g.M + T - 1) / T;
+  const int m0 = (blockIdx.x % tiles_m) * T, n0 = (blockIdx.x / tiles_m) * T;
+  const int KT = (g.K + BK - 1) / BK, kt0 = blockIdx.y * P.kt_per_split;
+  const int nkt = max(0, min(KT, kt0 + P.kt_per_split) - kt0);
+  const int krem = g.K - kt0 * BK;
+  const int k8 = 8 * (warp >> 2);                              // this group's half of a stage
+  const int wm = (warp & 1) * 16, wn = ((warp >> 1) & 1) * 16, fg = lane >> 2, ft = lane & 3;
+  double cr[2][4], ci[2][4];
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) cr[j][e] = ci[j][e] = 0.0;
 
-  const int KT = (g.K + BK - 1) / BK;
-  const int kt0 = split * P.kt_per_split;
-  const int kt1 = min(KT, kt0 + P.kt_per_split);
-  const int nkt = max(0, kt1 - kt0);
-
-  const int wm = (warp & 1) * 32, wn = (warp >> 1) * 32;
-  const int fg = lane >> 2, ft = lane & 3;   // fragment group / thread-in-group
-  // accumulators: 2 (16-row) x 4 (8-column) blocks of the warp's 32x32 tile
-  double cr[2][4][4], ci[2][4][4];
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) cr[i][j][e] = ci[i][j][e] = 0.0;
-
-  // prologue: STAGES-1 tiles in flight
-#pragma unroll
-  for (int s = 0; s < STAGES - 1; ++s) {
-    if (s < nkt) {
-      cd* st = smem + s * STAGE_ELEMS;
-      load_tile<A_MCONTIG, B_KCONTIG>(st, st + BK * LDA_S, A, B, g, m0, n0, (kt0 + s) * BK, tid);
+  Stream sa(g.A + (int64_t)blockIdx.z * g.a_b, g.a_m, g.a_k, m0, g.M, kt0 * BK, tid);
+  Stream sb(g.B + (int64_t)blockIdx.z * g.b_b, g.b_n, g.b_k, n0, g.N, kt0 * BK, tid);
+  auto refill = [&](int t) {
+    if (t < nkt) {
+      const unsigned st = su32(smem + (t % CP_STAGES) * STAGE);
+      sa.load(st, krem - t * BK);
+      sb.load(st + (unsigned)(BK * LDS * sizeof(cd)), krem - t * BK);
     }
     cp_async_commit();
-  }
+  };
+#pragma unroll
+  for (int t = 0; t < CP_STAGES - 1; ++t) refill(t);
+#pragma unroll 1
   for (int t = 0; t < nkt; ++t) {
-    cp_async_wait<STAGES - 2>();
+    cp_async_wait<CP_STAGES - 2>();
     __syncthreads();
-    {  // refill the stage consumed two iterations ago
-      const int tn = t + STAGES - 1;
-      if (tn < nkt) {
-        cd* st = smem + (tn % STAGES) * STAGE_ELEMS;
-        load_tile<A_MCONTIG, B_KCONTIG>(st, st + BK * LDA_S, A, B, g, m0, n0, (kt0 + tn) * BK, tid);
-      }
-      cp_async_commit();
-    }
-    const cd* As = smem + (t % STAGES) * STAGE_ELEMS;
-    const cd* Bs = As + BK * LDA_S;
+    refill(t + CP_STAGES - 1);   // the slot consumed in the last iteration
+    const cd* As = smem + (t % CP_STAGES) * STAGE + (k8 + ft) * LDS + wm + fg;
+    const cd* Bs = smem + (t % CP_STAGES) * STAGE + BK * LDS + (k8 + ft) * LDS + wn + fg;
+    cd a[4], b[2][2];
 #pragma unroll
-    for (int k8 = 0; k8 < BK; k8 += 8) {
-      double ar[2][4], ai[2][4], nai[2][4], br[4][2], bi[4][2];
+    for (int e = 0; e < 4; ++e) a[e] = As[4 * (e >> 1) * LDS + 8 * (e & 1)];
 #pragma unroll
-      for (int i = 0; i < 2; ++i)
+    for (int j = 0; j < 2; ++j)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const cd a = As[(k8 + ft + 4 * (e >> 1)) * LDA_S + wm + 16 * i + 8 * (e & 1) + fg];
-          ar[i][e] = a.x;
-          ai[i][e] = CONJA ? -a.y : a.y;
-          nai[i][e] = -ai[i][e];
-        }
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const cd bb = Bs[(k8 + ft + 4 * e) * LDB_S + wn + 8 * j + fg];
-          br[j][e] = bb.x;
-          bi[j][e] = CONJB ? -bb.y : bb.y;
-        }
-      // Re += Ar Br - Ai Bi, Im += Ar Bi + Ai Br, term-major so one accumulator's two
-      // products sit eight issues apart
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) dmma16(cr[i][j], ar[i], br[j]);
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) dmma16(ci[i][j], ar[i], bi[j]);
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) dmma16(cr[i][j], nai[i], bi[j]);
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) dmma16(ci[i][j], ai[i], br[j]);
-    }
+      for (int e = 0; e < 2; ++e) b[j][e] = Bs[4 * e * LDS + 8 * j];
+    mma_k8(cr, ci, a, b, CONJA, CONJB);
   }
   cp_async_wait<0>();
-
-  // accumulator (i, j, e): row wm + 16i + 8(e/2) + fg, column wn + 8j + 2ft + e%2
-  if (P.splits > 1) {
-    cd* W = P.ws + ((int64_t)split * g.batch + b) * (int64_t)g.M * g.N;
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int m = m0 + wm + 16 * i + 8 * (e >> 1) + fg;
-          const int n = n0 + wn + 8 * j + 2 * ft + (e & 1);
-          if (m < g.M && n < g.N) W[(int64_t)n * g.M + m] = cmk(cr[i][j][e], ci[i][j][e]);
-        }
-    return;
-  }
-  cd* C = g.C + (int64_t)b * g.c_b;
-  const bool use_beta = (g.beta.x != 0.0) || (g.beta.y != 0.0);
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int m = m0 + wm + 16 * i + 8 * (e >> 1) + fg;
-        const int n = n0 + wn + 8 * j + 2 * ft + (e & 1);
-        if (m >= g.M || n >= g.N) continue;
-        cd* c = C + (int64_t)m * g.c_m + (int64_t)n * g.c_n;
-        cd v = cmul(g.alpha, cmk(cr[i][j][e], ci[i][j][e]));
-        if (use_beta) v = cadd(v, cmul(g.beta, *c));
-        *c = v;
-      }
-}
-
-__global__ void splitk_reduce_kernel(Gemm g, int splits, const cd* __restrict__ ws) {
-  const int64_t MN = (int64_t)g.M * g.N;
-  const int64_t total = MN * g.batch;
-  const bool use_beta = (g.beta.x != 0.0) || (g.beta.y != 0.0);
-  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    int64_t b = idx / MN, r = idx % MN;
-    int m = (int)(r % g.M), n = (int)(r / g.M);
-    cd s = cmk(0.0, 0.0);
-    for (int q = 0; q < splits; ++q) s = cadd(s, ws[((int64_t)q * g.batch + b) * MN + r]);
-    cd* c = g.C + b * g.c_b + (int64_t)m * g.c_m + (int64_t)n * g.c_n;
-    cd v = cmul(g.alpha, s);
-    if (use_beta) v = cadd(v, cmul(g.beta, *c));
-    *c = v;
-  }
+  __syncthreads();   // every warp is done with the stages
+  finish_tile(P, smem, cr, ci, m0, n0);
 }
 
 __global__ void scale_c_kernel(Gemm g) {
@@ -225,18 +322,60 @@ __global__ void scale_c_kernel(Gemm g) {
   }
 }
 
-typedef void (*KernelFn)(GemmParams);
+typedef void (*CopyKernel)(GemmParams);
+typedef void (*TmaKernel)(const CUtensorMap, const CUtensorMap, GemmParams);
 
 template <bool CA, bool CB>
-KernelFn pick_layout(bool amc, bool bkc) {
-  if (amc) return bkc ? zgemm_kernel<CA, CB, true, true> : zgemm_kernel<CA, CB, true, false>;
-  return bkc ? zgemm_kernel<CA, CB, false, true> : zgemm_kernel<CA, CB, false, false>;
+TmaKernel pick_layout(bool amc, bool bkc) {
+  if (amc) return bkc ? zgemm_tma_kernel<CA, CB, true, true> : zgemm_tma_kernel<CA, CB, true, false>;
+  return bkc ? zgemm_tma_kernel<CA, CB, false, true> : zgemm_tma_kernel<CA, CB, false, false>;
 }
-
-KernelFn pick(const Gemm& g) {
-  bool amc = (g.a_m == 1), bkc = (g.b_k == 1);
+TmaKernel pick_tma(const Gemm& g, bool amc, bool bkc) {
   if (g.conjA) return g.conjB ? pick_layout<true, true>(amc, bkc) : pick_layout<true, false>(amc, bkc);
   return g.conjB ? pick_layout<false, true>(amc, bkc) : pick_layout<false, false>(amc, bkc);
+}
+CopyKernel pick_copy(const Gemm& g) {
+  if (g.conjA) return g.conjB ? zgemm_copy_kernel<true, true> : zgemm_copy_kernel<true, false>;
+  return g.conjB ? zgemm_copy_kernel<false, true> : zgemm_copy_kernel<false, false>;
+}
+
+// The tensor map of an operand (free x K, copies s_b apart), as doubles: the contiguous index (two
+// doubles an element), the other one, the copy.  False when a map does not describe it.
+bool operand_map(CUtensorMap* map, const cd* p, int64_t extent, int64_t s_free, int64_t K, int64_t s_k, int batch, int64_t s_b,
+                 bool* free_contig) {
+  // an index of extent 1 is contiguous whatever its stride
+  *free_contig = s_free == 1 || (extent == 1 && s_k != 1);
+  if (!*free_contig && s_k != 1 && K != 1) return false;
+  const int64_t n0 = *free_contig ? extent : K, n1 = *free_contig ? K : extent;
+  int64_t s1 = *free_contig ? s_k : s_free;
+  if (n1 == 1) s1 = n0;
+  if (s_b == 0) { batch = 1; s_b = 1; }
+  const int64_t most = (int64_t)1 << 35;   // strides below 2^40 bytes, extents below 2^32
+  if (s1 < 1 || s1 >= most || s_b < 1 || s_b >= most || (reinterpret_cast<uintptr_t>(p) & 15)) return false;
+  cuuint64_t dims[3] = {(cuuint64_t)(2 * n0), (cuuint64_t)n1, (cuuint64_t)batch};
+  cuuint64_t strides[2] = {(cuuint64_t)s1 * sizeof(cd), (cuuint64_t)s_b * sizeof(cd)};
+  cuuint32_t box[3] = {16, (cuuint32_t)(*free_contig ? BK : T), 1}, estr[3] = {1, 1, 1};
+  const auto encode = tensor_map_encoder();
+  return encode && encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, const_cast<cd*>(p), dims, strides, box, estr,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// K splits for `tiles` tiles of KT stages.  Measured on a B200: a stage takes 1475 clocks in a CTA alone
+// on its SM and 1090 (the FP64 tensor pipe's rate) beside others; a CTA costs 3000 clocks around its
+// stages, 5000 with the cluster's sum, about half of it hidden behind its SM's other CTAs.  E.g. 128 x
+// 512 x 1024 (64 tiles): 51.2 / 28.8 / 26.7 / 32.9 us at 1 / 2 / 4 / 8 splits; 512 x 1024 x 128 (512
+// tiles) 30.4 / 32.5 / 42.2.
+int choose_splits(double tiles, int KT) {
+  int best = 1;
+  double tbest = 1e300;
+  for (int s = 1; s <= SPLIT_MAX && (s == 1 || KT >= 2 * s); ++s) {
+    const double w = std::ceil(tiles * s / 148.0), stages = (KT + s - 1) / s;
+    const double ov = s > 1 ? 5000.0 : 3000.0;
+    const double t = w <= 1.0 ? stages * 1475.0 + ov : w * stages * 1090.0 + ov * (1.0 + 0.5 * (w - 1.0));
+    if (t < tbest) { tbest = t; best = s; }
+  }
+  return best;
 }
 
 }  // namespace
@@ -253,43 +392,38 @@ int gemm_launch(const Gemm& g, Workspace* ws, cudaStream_t s) {
     MPSB_CUDA_TRY(cudaGetLastError());
     return MPSB_OK;
   }
-  const int tiles = ((g.M + BM - 1) / BM) * ((g.N + BN - 1) / BN);
-  const int KT = (g.K + BK - 1) / BK;
-  const int64_t ctas = (int64_t)tiles * g.batch;
-  int splits = 1;
-  const int target = 2 * 148;  // two resident 64x64 tiles per SM
-  // without a workspace (ws == nullptr) K is never split, so no scratch is needed
-  // splits of at least two K tiles (measured on the RK4 step, 40 sites at chi=128, d=4:
-  // 87.4 ms with >= 4 tiles per split from KT >= 8, 82.7 ms with >= 2 from KT >= 4)
-  const int64_t basis = (ws && ws->per_problem) ? (int64_t)tiles : ctas;
-  if (ws && basis < target && KT >= 4) {
-    splits = (int)std::min<int64_t>((target + basis - 1) / basis, KT / 2);
-    splits = std::max(1, std::min(splits, 32));
-  }
-  int kt_per = (KT + splits - 1) / splits;
-  splits = (KT + kt_per - 1) / kt_per;
-
+  // without a workspace (ws == nullptr) K is not split
+  const int tiles = ((g.M + T - 1) / T) * ((g.N + T - 1) / T), KT = (g.K + BK - 1) / BK;
+  // in batched mode the partition must not depend on the number of copies: it is that of four, the
+  // usual bucket's order (the copies fill the chip, so splitting for one only adds sums)
+  int splits = ws ? choose_splits((double)tiles * (ws->per_problem ? 4 : g.batch), KT) : 1;
   GemmParams P;
   P.g = g;
-  P.splits = splits;
-  P.kt_per_split = kt_per;
-  P.ws = nullptr;
-  if (splits > 1) {
-    size_t bytes = (size_t)splits * g.batch * g.M * g.N * sizeof(cd);
-    MPSB_TRY(ws_splitk(ws, bytes, &P.ws));
-  }
-  KernelFn fn = pick(g);
-  MPSB_TRY(ensure_kernel_attrs((const void*)fn, (int)SMEM_BYTES));
-  dim3 grid(tiles, splits, g.batch);
-  fn<<<grid, NT, SMEM_BYTES, s>>>(P);
-  MPSB_CUDA_TRY(cudaGetLastError());
-  if (splits > 1) {
-    count_launch(ws);
-    int64_t total = (int64_t)g.M * g.N * g.batch;
-    int blocks = (int)std::min<int64_t>((total + 255) / 256, 148 * 8);
-    splitk_reduce_kernel<<<blocks, 256, 0, s>>>(g, splits, P.ws);
-    MPSB_CUDA_TRY(cudaGetLastError());
-  }
+  P.kt_per_split = (KT + splits - 1) / splits;
+  splits = (KT + P.kt_per_split - 1) / P.kt_per_split;
+  P.err = ws ? ws->err : nullptr;
+  CUtensorMap ma, mb;
+  bool amc, bnc;
+  const bool tma = operand_map(&ma, g.A, g.M, g.a_m, g.K, g.a_k, g.batch, g.a_b, &amc) &&
+                   operand_map(&mb, g.B, g.N, g.b_n, g.K, g.b_k, g.batch, g.b_b, &bnc);
+  const TmaKernel tk = tma ? pick_tma(g, amc, !bnc) : nullptr;
+  const CopyKernel ck = tma ? nullptr : pick_copy(g);
+  const size_t smem = tma ? SMEM_TMA : SMEM_COPY;
+  MPSB_TRY(ensure_kernel_attrs(tma ? (const void*)tk : (const void*)ck, (int)smem, true));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(tiles, splits, g.batch);
+  cfg.blockDim = dim3(NT, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = splits;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = splits > 1 ? 1 : 0;
+  if (tma) MPSB_CUDA_TRY(cudaLaunchKernelEx(&cfg, tk, ma, mb, P));
+  else MPSB_CUDA_TRY(cudaLaunchKernelEx(&cfg, ck, P));
   return MPSB_OK;
 }
 

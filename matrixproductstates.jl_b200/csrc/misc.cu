@@ -6,6 +6,7 @@
 
 #include "common.cuh"
 #include "misc.cuh"
+#include "tma.cuh"
 
 namespace mpsb {
 
@@ -21,6 +22,18 @@ int ensure_kernel_attrs(const void* fn, int smem_bytes, bool cluster16) {
   done.insert({dev, fn});
   return MPSB_OK;
 }
+
+PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
+  static const PFN_cuTensorMapEncodeTiled_v12000 encode = [] {
+    cudaDriverEntryPointQueryResult q;
+    void* fn = nullptr;
+    const bool ok = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) == cudaSuccess &&
+                    q == cudaDriverEntryPointSuccess;
+    return ok ? reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn) : nullptr;
+  }();
+  return encode;
+}
+
 namespace {
 
 __global__ void set_value_kernel(cd* p, cd v) { *p = v; }

@@ -37,6 +37,7 @@
 
 #include "common.cuh"
 #include "ozaki.cuh"
+#include "tma.cuh"
 #include "workspace.cuh"
 
 namespace mpsb {
@@ -604,31 +605,18 @@ __global__ void wait_probe_kernel(unsigned long long limit_ns, int* err) {
 }
 
 // ---------------------------------------------------------------- host side
-PFN_cuTensorMapEncodeTiled_v12000 g_encode = nullptr;
-std::once_flag g_encode_once;
-
-int get_encoder() {
-  std::call_once(g_encode_once, [] {
-    cudaDriverEntryPointQueryResult q;
-    void* fn = nullptr;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      g_encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
-  });
-  if (!g_encode) {
-    set_last_message("cuTensorMapEncodeTiled is not available from the driver");
-    return MPSB_ERR_CUDA;
-  }
-  return MPSB_OK;
-}
-
 // 2-d int8 tensor map of a slice buffer (rows of kp bytes), tiles of 64 bytes x box_rows
 int make_map(CUtensorMap* map, const int8_t* base, int64_t kp, int64_t rows, int box_rows) {
   cuuint64_t dims[2] = {(cuuint64_t)kp, (cuuint64_t)rows};
   cuuint64_t strides[1] = {(cuuint64_t)kp};
   cuuint32_t box[2] = {(cuuint32_t)OZ_BK, (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1, 1};
-  CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<int8_t*>(base), dims, strides, box, estr,
+  const PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
+  if (!encode) {
+    set_last_message("cuTensorMapEncodeTiled is not available from the driver");
+    return MPSB_ERR_CUDA;
+  }
+  CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<int8_t*>(base), dims, strides, box, estr,
                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
@@ -731,7 +719,6 @@ int ozgemm_launch(const Gemm& g, int slices, void* scratch, size_t scratch_bytes
                   cudaStream_t s) {
   if (!ozgemm_supported(g, slices)) return MPSB_ERR_UNSUPPORTED;
   if (scratch_bytes < ozgemm_scratch_bytes(g, slices)) return MPSB_ERR_INVALID_ARG;
-  MPSB_TRY(get_encoder());
   const int S = slices;
   const int64_t Mpad = round_up(g.M, OZ_BM), NBpad = round_up(2 * (int64_t)g.N, OZ_BN);
   const int64_t Kp = round_up(2 * (int64_t)g.K, OZ_KP_ALIGN);

@@ -984,6 +984,7 @@ int qr_blocked(const QrProblem& p, Workspace* ws, cudaStream_t s) {
   Workspace* sw = ws->qr_side_ws;
   sw->capturing = ws->capturing;
   sw->per_problem = ws->per_problem;
+  sw->err = ws->err;
   cudaStream_t ls = ws->qr_side;
   cudaEvent_t ev_v = ws->qr_ev[0], ev_t = ws->qr_ev[1];
   cd* Vb = static_cast<cd*>(ws->qr.p);

@@ -14,13 +14,13 @@ struct DevBuf {
 };
 
 struct Workspace {
-  DevBuf splitk;          // split-K partial tiles
+  int* err = nullptr;     // the context's device error word
   DevBuf qr;              // QR: the panels' T; blocked form also reflectors, V^H V and T V1^H
   DevBuf svd;             // SVD: the Jacobi working matrix, V, norms, flags
   DevBuf oz;              // sliced tensor-core GEMM: int8 slices of both operands, row exponents
   DevBuf named[16];       // per-sweep temporaries (see engine.cu)
   bool capturing = false;
-  // batched calls: a GEMM's split-K partition is chosen from one problem's shape alone (not
+  // batched calls: a GEMM's K split is chosen from one problem's shape alone (not
   // from the batch's grid), so every copy of a batch computes exactly what the same problem
   // computes in a batch of one
   bool per_problem = false;
@@ -33,7 +33,7 @@ struct Workspace {
   };
   std::vector<TimedLaunch>* prof = nullptr;
   // look-ahead lane of the blocked QR (created by its first eager call): a stream, the two events
-  // of its fork / join, and the lane's own workspace (its GEMMs' split-K partials)
+  // of its fork / join, and the lane's own workspace
   cudaStream_t qr_side = nullptr;
   cudaEvent_t qr_ev[2] = {nullptr, nullptr};
   Workspace* qr_side_ws = nullptr;
@@ -79,7 +79,7 @@ inline void ws_free(Workspace& w) {
     delete w.qr_side_ws;
     w.qr_side_ws = nullptr;
   }
-  DevBuf* all[] = {&w.splitk, &w.qr, &w.svd, &w.oz};
+  DevBuf* all[] = {&w.qr, &w.svd, &w.oz};
   for (DevBuf* b : all) {
     if (b->p) cudaFree(b->p);
     b->p = nullptr;
@@ -90,13 +90,6 @@ inline void ws_free(Workspace& w) {
     b.p = nullptr;
     b.cap = 0;
   }
-}
-
-inline int ws_splitk(Workspace* ws, size_t bytes, cd** out) {
-  if (!ws) return MPSB_ERR_INVALID_ARG;
-  MPSB_TRY(devbuf_ensure(ws, ws->splitk, bytes));
-  *out = static_cast<cd*>(ws->splitk.p);
-  return MPSB_OK;
 }
 
 }  // namespace mpsb
