@@ -92,6 +92,10 @@ struct Gemm {
 struct Workspace;  // device scratch owned by a context (engine.cu)
 
 int gemm_launch(const Gemm& g, Workspace* ws, cudaStream_t s);
+// Up to GEMM_GROUP problems (of one batch count) in one launch: each into its own C, or, when `sum`, all
+// into g[0].C = alpha sum_q A_q B_q + beta C (one M, N, C, alpha and beta: g[0]'s).
+constexpr int GEMM_GROUP = 4;
+int gemm_group_launch(const Gemm* g, int n, bool sum, Workspace* ws, cudaStream_t s);
 
 // Small-K "apply a local MPO tensor" contraction:
 //   Out[x, m, y] = sum_k In[x, k, y] * Op[k, m]   with k = (k1, k2), m = (m1, m2) split indices.

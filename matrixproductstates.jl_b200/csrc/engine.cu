@@ -87,7 +87,10 @@ static bool split_worth(const mpsb_ctx* ctx, const Gemm& g) {
   return tiles >= ctx->split_min_tiles && g.K >= 16;
 }
 
-int run_gemm(mpsb_ctx* ctx, const Gemm& g0) {
+static const cd ONE = {1.0, 0.0};
+static const cd ZERO = {0.0, 0.0};
+
+static Gemm with_copies(mpsb_ctx* ctx, const Gemm& g0) {
   Gemm g = g0;
   if (ctx->batch > 1 && g.batch == 1) {
     g.batch = ctx->batch;
@@ -95,13 +98,66 @@ int run_gemm(mpsb_ctx* ctx, const Gemm& g0) {
     g.b_b = ctx->stride_of(g.B);
     g.c_b = ctx->stride_of(g.C);
   }
-  if (ctx->split_on && ozgemm_supported(g, ctx->split_slices) && split_worth(ctx, g)) {
-    void* before_oz = ctx->ws.oz.p;
-    MPSB_TRY(devbuf_ensure(&ctx->ws, ctx->ws.oz, ozgemm_scratch_bytes(g, ctx->split_slices)));
-    if (ctx->ws.oz.p != before_oz) ctx->ws_generation++;
-    return ozgemm_launch(g, ctx->split_slices, ctx->ws.oz.p, ctx->ws.oz.cap, ctx->err(), &ctx->ws, ctx->stream);
+  return g;
+}
+
+static bool takes_split(const mpsb_ctx* ctx, const Gemm& g) {
+  return ctx->split_on && ozgemm_supported(g, ctx->split_slices) && split_worth(ctx, g);
+}
+
+static int run_split(mpsb_ctx* ctx, const Gemm& g) {
+  void* before_oz = ctx->ws.oz.p;
+  MPSB_TRY(devbuf_ensure(&ctx->ws, ctx->ws.oz, ozgemm_scratch_bytes(g, ctx->split_slices)));
+  if (ctx->ws.oz.p != before_oz) ctx->ws_generation++;
+  return ozgemm_launch(g, ctx->split_slices, ctx->ws.oz.p, ctx->ws.oz.cap, ctx->err(), &ctx->ws, ctx->stream);
+}
+
+int run_gemm(mpsb_ctx* ctx, const Gemm& g0) {
+  const Gemm g = with_copies(ctx, g0);
+  return takes_split(ctx, g) ? run_split(ctx, g) : gemm_launch(g, &ctx->ws, ctx->stream);
+}
+
+// Independent GEMMs of one site in as few launches as they fit; those that take the sliced path go
+// on their own.
+static int run_gemms(mpsb_ctx* ctx, const Gemm* list, int n) {
+  Gemm grp[GEMM_GROUP];
+  int m = 0;
+  for (int i = 0; i <= n; ++i) {
+    if (m == GEMM_GROUP || (i == n && m > 0)) {
+      MPSB_TRY(gemm_group_launch(grp, m, false, &ctx->ws, ctx->stream));
+      m = 0;
+    }
+    if (i == n) break;
+    const Gemm g = with_copies(ctx, list[i]);
+    if (takes_split(ctx, g)) MPSB_TRY(run_split(ctx, g));
+    else grp[m++] = g;
   }
-  return gemm_launch(g, &ctx->ws, ctx->stream);
+  return MPSB_OK;
+}
+
+// C = sum of the GEMMs (one shape and place of C), likewise.
+static int run_gemm_sum(mpsb_ctx* ctx, const Gemm* list, int n) {
+  Gemm grp[GEMM_GROUP], sliced[2 * GEMM_GROUP + 1];
+  int m = 0, ns = 0;
+  bool first = true;
+  auto place = [&](Gemm g) {
+    g.beta = first ? ZERO : ONE;
+    first = false;
+    return g;
+  };
+  for (int i = 0; i <= n; ++i) {
+    if (m == GEMM_GROUP || (i == n && m > 0)) {
+      grp[0] = place(grp[0]);
+      MPSB_TRY(gemm_group_launch(grp, m, true, &ctx->ws, ctx->stream));
+      m = 0;
+    }
+    if (i == n) break;
+    const Gemm g = with_copies(ctx, list[n - 1 - i]);   // the operator's term, the longest, first
+    if (takes_split(ctx, g)) sliced[ns++] = g;
+    else grp[m++] = g;
+  }
+  for (int i = 0; i < ns; ++i) MPSB_TRY(run_split(ctx, place(sliced[i])));
+  return MPSB_OK;
 }
 
 static inline int run_mpo(mpsb_ctx* ctx, const MpoApply& a0, int64_t k1, int64_t k2, int64_t m1, int64_t m2) {
@@ -116,12 +172,8 @@ static inline int run_mpo(mpsb_ctx* ctx, const MpoApply& a0, int64_t k1, int64_t
   return mpo_apply_launch_strided(a, k1, k2, m1, m2, ctx->stream);
 }
 
-static const cd ONE = {1.0, 0.0};
-static const cd ZERO = {0.0, 0.0};
-
 // prod_AOR (src/mps_base.jl:7-19): T = A*R (GEMM), AOR = O . T (small-K apply, permutes folded)
-int op_prod_AOR(mpsb_ctx* ctx, const cd* A, const cd* O, const cd* R, cd* AOR, int chiL, int d, int chiR, int wL,
-                int wR, int chiR0) {
+static int gemm_AR(mpsb_ctx* ctx, const cd* A, const cd* R, int chiL, int d, int chiR, int wR, int chiR0, Gemm* out) {
   cd* T;
   MPSB_TRY(ensure_slot(ctx, SLOT_T, (size_t)chiL * d * wR * chiR0 * sizeof(cd), &T));
   Gemm g;
@@ -129,7 +181,11 @@ int op_prod_AOR(mpsb_ctx* ctx, const cd* A, const cd* O, const cd* R, cd* AOR, i
   g.A = A; g.a_m = 1; g.a_k = (int64_t)chiL * d;
   g.B = R; g.b_k = 1; g.b_n = chiR;
   g.C = T; g.c_m = 1; g.c_n = (int64_t)chiL * d;
-  MPSB_TRY(run_gemm(ctx, g));
+  *out = g;
+  return MPSB_OK;
+}
+
+static int mpo_AOR(mpsb_ctx* ctx, const cd* T, const cd* O, cd* AOR, int chiL, int d, int wL, int wR, int chiR0) {
   MpoApply a;
   a.X = chiL; a.Y = chiR0; a.K1 = d; a.K2 = wR; a.M1 = wL; a.M2 = d;
   a.in = T; a.in_x = 1; a.in_k1 = chiL; a.in_k2 = (int64_t)chiL * d; a.in_y = (int64_t)chiL * d * wR;
@@ -138,9 +194,16 @@ int op_prod_AOR(mpsb_ctx* ctx, const cd* A, const cd* O, const cd* R, cd* AOR, i
   return run_mpo(ctx, a, (int64_t)wL * d * wR, (int64_t)wL * d, 1, wL);
 }
 
+int op_prod_AOR(mpsb_ctx* ctx, const cd* A, const cd* O, const cd* R, cd* AOR, int chiL, int d, int chiR, int wL,
+                int wR, int chiR0) {
+  Gemm g;
+  MPSB_TRY(gemm_AR(ctx, A, R, chiL, d, chiR, wR, chiR0, &g));
+  MPSB_TRY(run_gemm(ctx, g));
+  return mpo_AOR(ctx, g.C, O, AOR, chiL, d, wL, wR, chiR0);
+}
+
 // prod_AOL (src/mps_base.jl:26-39): G1 = L' * A (GEMM), AOL = G1 . O
-int op_prod_AOL(mpsb_ctx* ctx, const cd* A, const cd* O, const cd* L, cd* AOL, int chiL, int d, int chiR, int wL,
-                int wR, int chiL0) {
+static int gemm_LA(mpsb_ctx* ctx, const cd* A, const cd* L, int chiL, int d, int chiR, int wL, int chiL0, Gemm* out) {
   cd* G1;
   MPSB_TRY(ensure_slot(ctx, SLOT_G1, (size_t)wL * chiL0 * d * chiR * sizeof(cd), &G1));
   Gemm g;
@@ -148,7 +211,11 @@ int op_prod_AOL(mpsb_ctx* ctx, const cd* A, const cd* O, const cd* L, cd* AOL, i
   g.A = L; g.a_m = chiL; g.a_k = 1; g.conjA = true;
   g.B = A; g.b_k = 1; g.b_n = chiL;
   g.C = G1; g.c_m = 1; g.c_n = (int64_t)wL * chiL0;
-  MPSB_TRY(run_gemm(ctx, g));
+  *out = g;
+  return MPSB_OK;
+}
+
+static int mpo_AOL(mpsb_ctx* ctx, const cd* G1, const cd* O, cd* AOL, int d, int chiR, int wL, int wR, int chiL0) {
   MpoApply a;
   a.X = chiL0; a.Y = chiR; a.K1 = wL; a.K2 = d; a.M1 = d; a.M2 = wR;
   a.in = G1; a.in_x = wL; a.in_k1 = 1; a.in_k2 = (int64_t)wL * chiL0; a.in_y = (int64_t)wL * chiL0 * d;
@@ -157,54 +224,73 @@ int op_prod_AOL(mpsb_ctx* ctx, const cd* A, const cd* O, const cd* L, cd* AOL, i
   return run_mpo(ctx, a, 1, (int64_t)wL * d * wR, wL, (int64_t)wL * d);
 }
 
+int op_prod_AOL(mpsb_ctx* ctx, const cd* A, const cd* O, const cd* L, cd* AOL, int chiL, int d, int chiR, int wL,
+                int wR, int chiL0) {
+  Gemm g;
+  MPSB_TRY(gemm_LA(ctx, A, L, chiL, d, chiR, wL, chiL0, &g));
+  MPSB_TRY(run_gemm(ctx, g));
+  return mpo_AOL(ctx, g.C, O, AOL, d, chiR, wL, wR, chiL0);
+}
+
 // prod_LR!(A0, L, AOR) (src/mps_base.jl:53-61): A0 = L' * AOR
-int op_prod_LR_3_4(mpsb_ctx* ctx, const cd* L, const cd* AOR, cd* A0, int chiL, int wL, int chiL0, int d, int chiR0,
-                   cd alpha, cd beta) {
+static Gemm gemm_LR_3_4(const cd* L, const cd* AOR, cd* A0, int chiL, int wL, int chiL0, int d, int chiR0, cd alpha, cd beta) {
   Gemm g;
   g.M = chiL0; g.N = d * chiR0; g.K = chiL * wL;
   g.A = L; g.a_m = (int64_t)chiL * wL; g.a_k = 1; g.conjA = true;
   g.B = AOR; g.b_k = 1; g.b_n = (int64_t)chiL * wL;
   g.C = A0; g.c_m = 1; g.c_n = chiL0;
   g.alpha = alpha; g.beta = beta;
-  return run_gemm(ctx, g);
+  return g;
+}
+int op_prod_LR_3_4(mpsb_ctx* ctx, const cd* L, const cd* AOR, cd* A0, int chiL, int wL, int chiL0, int d, int chiR0,
+                   cd alpha, cd beta) {
+  return run_gemm(ctx, gemm_LR_3_4(L, AOR, A0, chiL, wL, chiL0, d, chiR0, alpha, beta));
 }
 
 // prod_LR!(A0, AOL, R) (src/mps_base.jl:73-81): A0 = AOL * R
-int op_prod_LR_4_3(mpsb_ctx* ctx, const cd* AOL, const cd* R, cd* A0, int chiL0, int d, int chiR, int wR, int chiR0,
-                   cd alpha, cd beta) {
+static Gemm gemm_LR_4_3(const cd* AOL, const cd* R, cd* A0, int chiL0, int d, int chiR, int wR, int chiR0, cd alpha, cd beta) {
   Gemm g;
   g.M = chiL0 * d; g.N = chiR0; g.K = chiR * wR;
   g.A = AOL; g.a_m = 1; g.a_k = (int64_t)chiL0 * d;
   g.B = R; g.b_k = 1; g.b_n = (int64_t)chiR * wR;
   g.C = A0; g.c_m = 1; g.c_n = (int64_t)chiL0 * d;
   g.alpha = alpha; g.beta = beta;
-  return run_gemm(ctx, g);
+  return g;
+}
+int op_prod_LR_4_3(mpsb_ctx* ctx, const cd* AOL, const cd* R, cd* A0, int chiL0, int d, int chiR, int wR, int chiR0,
+                   cd alpha, cd beta) {
+  return run_gemm(ctx, gemm_LR_4_3(AOL, R, A0, chiL0, d, chiR, wR, chiR0, alpha, beta));
 }
 
 // update_re!(env, A0, AOR) (src/mps_base.jl:151-160): env = AOR * A0'
-int op_update_re(mpsb_ctx* ctx, const cd* A0, const cd* AOR, cd* env, int chiL, int wL, int d, int chiR0, int chiL0) {
+static Gemm gemm_update_re(const cd* A0, const cd* AOR, cd* env, int chiL, int wL, int d, int chiR0, int chiL0) {
   Gemm g;
   g.M = chiL * wL; g.N = chiL0; g.K = d * chiR0;
   g.A = AOR; g.a_m = 1; g.a_k = (int64_t)chiL * wL;
   g.B = A0; g.b_k = chiL0; g.b_n = 1; g.conjB = true;
   g.C = env; g.c_m = 1; g.c_n = (int64_t)chiL * wL;
-  return run_gemm(ctx, g);
+  return g;
+}
+int op_update_re(mpsb_ctx* ctx, const cd* A0, const cd* AOR, cd* env, int chiL, int wL, int d, int chiR0, int chiL0) {
+  return run_gemm(ctx, gemm_update_re(A0, AOR, env, chiL, wL, d, chiR0, chiL0));
 }
 
 // update_le!(env, A0, AOL) (src/mps_base.jl:232-241): env = AOL' * A0
-int op_update_le(mpsb_ctx* ctx, const cd* A0, const cd* AOL, cd* env, int chiL0, int d, int chiR, int wR, int chiR0) {
+static Gemm gemm_update_le(const cd* A0, const cd* AOL, cd* env, int chiL0, int d, int chiR, int wR, int chiR0) {
   Gemm g;
   g.M = chiR * wR; g.N = chiR0; g.K = chiL0 * d;
   g.A = AOL; g.a_m = (int64_t)chiL0 * d; g.a_k = 1; g.conjA = true;
   g.B = A0; g.b_k = 1; g.b_n = (int64_t)chiL0 * d;
   g.C = env; g.c_m = 1; g.c_n = (int64_t)chiR * wR;
-  return run_gemm(ctx, g);
+  return g;
+}
+int op_update_le(mpsb_ctx* ctx, const cd* A0, const cd* AOL, cd* env, int chiL0, int d, int chiR, int wR, int chiR0) {
+  return run_gemm(ctx, gemm_update_le(A0, AOL, env, chiL0, d, chiR, wR, chiR0));
 }
 
 // prod_LR(L2, A3) (src/mps_base.jl:85-90, 100-108): out(x, rest) = L(x, chiL) * A(chiL, rest);
 // transL gives prod_LR_co (L.')
-int op_L2_A3(mpsb_ctx* ctx, const cd* L, const cd* A, cd* out, int x, int chiL, int rest, cd alpha, cd beta,
-             bool transL) {
+static Gemm gemm_L2_A3(const cd* L, const cd* A, cd* out, int x, int chiL, int rest, cd alpha, cd beta, bool transL) {
   Gemm g;
   g.M = x; g.N = rest; g.K = chiL;
   g.A = L;
@@ -212,39 +298,52 @@ int op_L2_A3(mpsb_ctx* ctx, const cd* L, const cd* A, cd* out, int x, int chiL, 
   g.B = A; g.b_k = 1; g.b_n = chiL;
   g.C = out; g.c_m = 1; g.c_n = x;
   g.alpha = alpha; g.beta = beta;
-  return run_gemm(ctx, g);
+  return g;
+}
+int op_L2_A3(mpsb_ctx* ctx, const cd* L, const cd* A, cd* out, int x, int chiL, int rest, cd alpha, cd beta,
+             bool transL) {
+  return run_gemm(ctx, gemm_L2_A3(L, A, out, x, chiL, rest, alpha, beta, transL));
 }
 
 // prod_LR(A3, R2) (src/mps_base.jl:122-137): out(lead, y) = A(lead, chiR) * R(chiR, y)
-int op_A3_R2(mpsb_ctx* ctx, const cd* A, const cd* R, cd* out, int lead, int chiR, int y, cd alpha, cd beta) {
+static Gemm gemm_A3_R2(const cd* A, const cd* R, cd* out, int lead, int chiR, int y, cd alpha, cd beta) {
   Gemm g;
   g.M = lead; g.N = y; g.K = chiR;
   g.A = A; g.a_m = 1; g.a_k = lead;
   g.B = R; g.b_k = 1; g.b_n = chiR;
   g.C = out; g.c_m = 1; g.c_n = lead;
   g.alpha = alpha; g.beta = beta;
-  return run_gemm(ctx, g);
+  return g;
+}
+int op_A3_R2(mpsb_ctx* ctx, const cd* A, const cd* R, cd* out, int lead, int chiR, int y, cd alpha, cd beta) {
+  return run_gemm(ctx, gemm_A3_R2(A, R, out, lead, chiR, y, alpha, beta));
 }
 
 // update_renv!(env, A0, AR) (src/mps_base.jl:193-199): env(chiA, chiL0) = AR(chiA, drest) * A0(chiL0, drest)'
-int op_update_renv(mpsb_ctx* ctx, const cd* A0, const cd* AR, cd* env, int chiA, int chiL0, int drest) {
+static Gemm gemm_update_renv(const cd* A0, const cd* AR, cd* env, int chiA, int chiL0, int drest) {
   Gemm g;
   g.M = chiA; g.N = chiL0; g.K = drest;
   g.A = AR; g.a_m = 1; g.a_k = chiA;
   g.B = A0; g.b_k = chiL0; g.b_n = 1; g.conjB = true;
   g.C = env; g.c_m = 1; g.c_n = chiA;
-  return run_gemm(ctx, g);
+  return g;
+}
+int op_update_renv(mpsb_ctx* ctx, const cd* A0, const cd* AR, cd* env, int chiA, int chiL0, int drest) {
+  return run_gemm(ctx, gemm_update_renv(A0, AR, env, chiA, chiL0, drest));
 }
 
 // update_lenv!(env, A0, AL) (src/mps_base.jl:275-281) and update_lenv_nc (:319-325):
 // env(chiR0, y) = A0(lead, chiR0)' * AL(lead, y)   (.' when !conj)
-int op_update_lenv(mpsb_ctx* ctx, const cd* A0, const cd* AL, cd* env, int lead, int chiR0, int y, bool conj) {
+static Gemm gemm_update_lenv(const cd* A0, const cd* AL, cd* env, int lead, int chiR0, int y, bool conj) {
   Gemm g;
   g.M = chiR0; g.N = y; g.K = lead;
   g.A = A0; g.a_m = lead; g.a_k = 1; g.conjA = conj;
   g.B = AL; g.b_k = 1; g.b_n = lead;
   g.C = env; g.c_m = 1; g.c_n = chiR0;
-  return run_gemm(ctx, g);
+  return g;
+}
+int op_update_lenv(mpsb_ctx* ctx, const cd* A0, const cd* AL, cd* env, int lead, int chiR0, int y, bool conj) {
+  return run_gemm(ctx, gemm_update_lenv(A0, AL, env, lead, chiR0, y, conj));
 }
 
 // QR through the context's workspace; a reallocated QR scratch invalidates captured graphs
@@ -351,6 +450,7 @@ static int sum_var_init(mpsb_ctx* ctx, bool right, mpsb_env* const* env, mpsb_en
   const mpsb_mps* AH = A[np];
   auto D = [&](int k) { return (int)Ain->dims[k]; };
   auto W = [&](int k) { return (int)H->w[k]; };
+  Gemm g[9];
   if (!right) {
     for (int l = 0; l < np; ++l) {
       MPSB_TRY(set_boundary(ctx, env[l]->entry(0), ONE));
@@ -360,12 +460,17 @@ static int sum_var_init(mpsb_ctx* ctx, bool right, mpsb_env* const* env, mpsb_en
     MPSB_TRY(set_boundary(ctx, envop->entry(na), coef[np]));
     for (int k = 0; k < na - 1; ++k) {
       if (wait) MPSB_CUDA_TRY(cudaStreamWaitEvent(ctx->stream, wait[k], 0));
-      for (int l = 0; l < np; ++l) {
-        MPSB_TRY(op_L2_A3(ctx, env[l]->entry(k), A[l]->site(k), s.P[l], D(k), D(k), d * D(k + 1), ONE, ZERO, false));
-        MPSB_TRY(op_update_lenv(ctx, Ain->site(k), s.P[l], env[l]->entry(k + 1), D(k) * d, D(k + 1), D(k + 1), true));
-      }
-      MPSB_TRY(op_prod_AOL(ctx, AH->site(k), H->site(k), envop->entry(k), s.AOL, D(k), d, D(k + 1), W(k), W(k + 1), D(k)));
-      MPSB_TRY(op_update_le(ctx, Ain->site(k), s.AOL, envop->entry(k + 1), D(k), d, D(k + 1), W(k + 1), D(k + 1)));
+      // every term's ket contraction, then every term's environment
+      for (int l = 0; l < np; ++l)
+        g[l] = gemm_L2_A3(env[l]->entry(k), A[l]->site(k), s.P[l], D(k), D(k), d * D(k + 1), ONE, ZERO, false);
+      MPSB_TRY(gemm_LA(ctx, AH->site(k), envop->entry(k), D(k), d, D(k + 1), W(k), D(k), &g[np]));
+      const cd* G1 = g[np].C;
+      MPSB_TRY(run_gemms(ctx, g, np + 1));
+      MPSB_TRY(mpo_AOL(ctx, G1, H->site(k), s.AOL, d, D(k + 1), W(k), W(k + 1), D(k)));
+      for (int l = 0; l < np; ++l)
+        g[l] = gemm_update_lenv(Ain->site(k), s.P[l], env[l]->entry(k + 1), D(k) * d, D(k + 1), D(k + 1), true);
+      g[np] = gemm_update_le(Ain->site(k), s.AOL, envop->entry(k + 1), D(k), d, D(k + 1), W(k + 1), D(k + 1));
+      MPSB_TRY(run_gemms(ctx, g, np + 1));
     }
   } else {
     for (int l = 0; l < np; ++l) {
@@ -376,12 +481,16 @@ static int sum_var_init(mpsb_ctx* ctx, bool right, mpsb_env* const* env, mpsb_en
     MPSB_TRY(set_boundary(ctx, envop->entry(0), coef[np]));
     for (int k = na - 1; k >= 1; --k) {
       if (wait) MPSB_CUDA_TRY(cudaStreamWaitEvent(ctx->stream, wait[k], 0));
-      for (int l = 0; l < np; ++l) {
-        MPSB_TRY(op_A3_R2(ctx, A[l]->site(k), env[l]->entry(k + 1), s.P[l], D(k) * d, D(k + 1), D(k + 1), ONE, ZERO));
-        MPSB_TRY(op_update_renv(ctx, Ain->site(k), s.P[l], env[l]->entry(k), D(k), D(k), d * D(k + 1)));
-      }
-      MPSB_TRY(op_prod_AOR(ctx, AH->site(k), H->site(k), envop->entry(k + 1), s.AOR, D(k), d, D(k + 1), W(k), W(k + 1), D(k + 1)));
-      MPSB_TRY(op_update_re(ctx, Ain->site(k), s.AOR, envop->entry(k), D(k), W(k), d, D(k + 1), D(k)));
+      for (int l = 0; l < np; ++l)
+        g[l] = gemm_A3_R2(A[l]->site(k), env[l]->entry(k + 1), s.P[l], D(k) * d, D(k + 1), D(k + 1), ONE, ZERO);
+      MPSB_TRY(gemm_AR(ctx, AH->site(k), envop->entry(k + 1), D(k), d, D(k + 1), W(k + 1), D(k + 1), &g[np]));
+      const cd* T = g[np].C;
+      MPSB_TRY(run_gemms(ctx, g, np + 1));
+      MPSB_TRY(mpo_AOR(ctx, T, H->site(k), s.AOR, D(k), d, W(k), W(k + 1), D(k + 1)));
+      for (int l = 0; l < np; ++l)
+        g[l] = gemm_update_renv(Ain->site(k), s.P[l], env[l]->entry(k), D(k), D(k), d * D(k + 1));
+      g[np] = gemm_update_re(Ain->site(k), s.AOR, envop->entry(k), D(k), W(k), d, D(k + 1), D(k));
+      MPSB_TRY(run_gemms(ctx, g, np + 1));
     }
   }
   return MPSB_OK;
@@ -399,34 +508,43 @@ static int sum_var_sweep(mpsb_ctx* ctx, bool right, mpsb_mps* A0, mpsb_env* cons
     if (rec) MPSB_CUDA_TRY(cudaEventRecord(rec[k], ctx->stream));
     return MPSB_OK;
   };
+  Gemm g[9];
   if (!right) {
     for (int k = na - 1; k >= 0; --k) {
       cd* out = A0->site(k);
-      for (int l = 0; l < np; ++l) {
-        MPSB_TRY(op_A3_R2(ctx, A[l]->site(k), env[l]->entry(k + 1), s.P[l], D(k) * d, D(k + 1), D(k + 1), ONE, ZERO));
-        MPSB_TRY(op_L2_A3(ctx, env[l]->entry(k), s.P[l], out, D(k), D(k), d * D(k + 1), ONE, l ? ONE : ZERO, false));
-      }
-      MPSB_TRY(op_prod_AOR(ctx, AH->site(k), H->site(k), envop->entry(k + 1), s.AOR, D(k), d, D(k + 1), W(k), W(k + 1), D(k + 1)));
-      MPSB_TRY(op_prod_LR_3_4(ctx, envop->entry(k), s.AOR, out, D(k), W(k), D(k), d, D(k + 1), ONE, np ? ONE : ZERO));
+      for (int l = 0; l < np; ++l)
+        g[l] = gemm_A3_R2(A[l]->site(k), env[l]->entry(k + 1), s.P[l], D(k) * d, D(k + 1), D(k + 1), ONE, ZERO);
+      MPSB_TRY(gemm_AR(ctx, AH->site(k), envop->entry(k + 1), D(k), d, D(k + 1), W(k + 1), D(k + 1), &g[np]));
+      const cd* T = g[np].C;
+      MPSB_TRY(run_gemms(ctx, g, np + 1));
+      MPSB_TRY(mpo_AOR(ctx, T, H->site(k), s.AOR, D(k), d, W(k), W(k + 1), D(k + 1)));
+      for (int l = 0; l < np; ++l)
+        g[l] = gemm_L2_A3(env[l]->entry(k), s.P[l], out, D(k), D(k), d * D(k + 1), ONE, ZERO, false);
+      g[np] = gemm_LR_3_4(envop->entry(k), s.AOR, out, D(k), W(k), D(k), d, D(k + 1), ONE, ZERO);
+      MPSB_TRY(run_gemm_sum(ctx, g, np + 1));
       if (k == 0) {
         MPSB_TRY(final_site(0));
         break;
       }
       MPSB_TRY(op_orth_right(ctx, out, D(k), d, D(k + 1)));
       MPSB_TRY(final_site(k));
-      for (int l = 0; l < np; ++l)
-        MPSB_TRY(op_update_renv(ctx, out, s.P[l], env[l]->entry(k), D(k), D(k), d * D(k + 1)));
-      MPSB_TRY(op_update_re(ctx, out, s.AOR, envop->entry(k), D(k), W(k), d, D(k + 1), D(k)));
+      for (int l = 0; l < np; ++l) g[l] = gemm_update_renv(out, s.P[l], env[l]->entry(k), D(k), D(k), d * D(k + 1));
+      g[np] = gemm_update_re(out, s.AOR, envop->entry(k), D(k), W(k), d, D(k + 1), D(k));
+      MPSB_TRY(run_gemms(ctx, g, np + 1));
     }
   } else {
     for (int k = 0; k < na; ++k) {
       cd* out = A0->site(k);
-      for (int l = 0; l < np; ++l) {
-        MPSB_TRY(op_L2_A3(ctx, env[l]->entry(k), A[l]->site(k), s.P[l], D(k), D(k), d * D(k + 1), ONE, ZERO, false));
-        MPSB_TRY(op_A3_R2(ctx, s.P[l], env[l]->entry(k + 1), out, D(k) * d, D(k + 1), D(k + 1), ONE, l ? ONE : ZERO));
-      }
-      MPSB_TRY(op_prod_AOL(ctx, AH->site(k), H->site(k), envop->entry(k), s.AOL, D(k), d, D(k + 1), W(k), W(k + 1), D(k)));
-      MPSB_TRY(op_prod_LR_4_3(ctx, s.AOL, envop->entry(k + 1), out, D(k), d, D(k + 1), W(k + 1), D(k + 1), ONE, np ? ONE : ZERO));
+      for (int l = 0; l < np; ++l)
+        g[l] = gemm_L2_A3(env[l]->entry(k), A[l]->site(k), s.P[l], D(k), D(k), d * D(k + 1), ONE, ZERO, false);
+      MPSB_TRY(gemm_LA(ctx, AH->site(k), envop->entry(k), D(k), d, D(k + 1), W(k), D(k), &g[np]));
+      const cd* G1 = g[np].C;
+      MPSB_TRY(run_gemms(ctx, g, np + 1));
+      MPSB_TRY(mpo_AOL(ctx, G1, H->site(k), s.AOL, d, D(k + 1), W(k), W(k + 1), D(k)));
+      for (int l = 0; l < np; ++l)
+        g[l] = gemm_A3_R2(s.P[l], env[l]->entry(k + 1), out, D(k) * d, D(k + 1), D(k + 1), ONE, ZERO);
+      g[np] = gemm_LR_4_3(s.AOL, envop->entry(k + 1), out, D(k), d, D(k + 1), W(k + 1), D(k + 1), ONE, ZERO);
+      MPSB_TRY(run_gemm_sum(ctx, g, np + 1));
       if (k == na - 1) {
         MPSB_TRY(final_site(k));
         break;
@@ -434,8 +552,9 @@ static int sum_var_sweep(mpsb_ctx* ctx, bool right, mpsb_mps* A0, mpsb_env* cons
       MPSB_TRY(op_orth_left(ctx, out, D(k), d, D(k + 1), nullptr));
       MPSB_TRY(final_site(k));
       for (int l = 0; l < np; ++l)
-        MPSB_TRY(op_update_lenv(ctx, out, s.P[l], env[l]->entry(k + 1), D(k) * d, D(k + 1), D(k + 1), true));
-      MPSB_TRY(op_update_le(ctx, out, s.AOL, envop->entry(k + 1), D(k), d, D(k + 1), W(k + 1), D(k + 1)));
+        g[l] = gemm_update_lenv(out, s.P[l], env[l]->entry(k + 1), D(k) * d, D(k + 1), D(k + 1), true);
+      g[np] = gemm_update_le(out, s.AOL, envop->entry(k + 1), D(k), d, D(k + 1), W(k + 1), D(k + 1));
+      MPSB_TRY(run_gemms(ctx, g, np + 1));
     }
   }
   return MPSB_OK;
