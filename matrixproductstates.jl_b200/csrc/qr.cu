@@ -35,9 +35,10 @@
 //     between warps through shared memory costs 160 clocks, an exchange between CTAs about 400, the
 //     reflector about 200 (FP64 latency 8 clocks, a shuffle 24), so the redundant arithmetic is cheaper.
 //   * the compact-WY factor T of a panel is built by a ninth warp, a column behind.
-//   * block reflectors: partials of V^H A on the FP64 tensor path, one bulk copy to the owner of
-//     each column slice, reduced there in a fixed order with T (or T^H) applied, the slice copied to
-//     every CTA, then A -= V W on the tensor path.
+//   * block reflectors: partials of V^H A on the FP64 tensor path, pushed to the owner of each column
+//     slice, reduced there in a fixed order with T (or T^H) applied, the slice pushed to every CTA,
+//     then A -= V W on the tensor path.  (Bulk copies in place of the pushes need a proxy fence per
+//     exchange, which took 1000 clocks.)
 //   * Q = H(1)...H(n) [I; 0] is formed in place in shared memory by applying the panels' block
 //     reflectors backwards to E (zungqr), so the matrix is read once and Q written once.
 // Reductions run in a fixed order, so every CTA and warp computes bit-identical reflectors and
@@ -52,8 +53,8 @@
 // FP64 tensor rate of the cluster's SMs.  One row per lane and many CTAs beat more rows per lane
 // (512 x 128 at 1 / 2 / 4 rows: 254 / 324 / 491 us) because the products scale with the CTAs.
 // Against the form with a reflector warp behind block barriers, Q as GEMMs over a back substitution
-// and outer panels of 16 columns (B200, Q only): 64 x 32 108.7 -> 51.2 us, 512 x 128 394 -> 254,
-// 512 x 256 818 -> 677, 2048 x 512 3990 -> 2510.
+// and outer panels of 16 columns (B200, Q only): 64 x 32 108.7 -> 50.2 us, 512 x 128 394 -> 248,
+// 512 x 256 818 -> 635, 2048 x 512 3990 -> 2140.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -74,9 +75,9 @@ constexpr int NT = 32 * (NWM + 1);     // and the warp that builds T
 constexpr int CMAX = 16;
 constexpr size_t SMEM_LIMIT = 227 * 1024;
 constexpr int WAIT_LIMIT = 1 << 20;
-constexpr int LDT = NB + 1, LDR = NB + 1, LDW = NB + 1;   // leading dimensions of T, the exchanged partials, the gathered W
+constexpr int LDT = NB + 1, LDW = NB + 1;   // leading dimensions of T, the gathered W
 enum { MB_COL = 0, MB_RS = 2, MB_AG, MB_COUNT };
-constexpr int BAR_PANEL = 1, BAR_TILES = 2, BAR_END = 3;   // named barriers: a step (C == 1), the product warps, a panel's end
+constexpr int BAR_PANEL = 1, BAR_END = 2;   // named barriers: a step (C == 1), a panel's end
 
 struct QrParams {
   QrProblem p;
@@ -90,7 +91,7 @@ struct QrParams {
   int64_t t_ld, t_b;
   int C, npanels, ldS, nc, ksc;   // nc: columns per exchange of a block reflector, ksc = ceil(nc / C)
   // shared-memory offsets (complex elements) and the byte offset of the mbarriers
-  int o_S, o_V, o_col, o_rcol, o_stg, o_rrs, o_w2s, o_w2o, o_rag, o_T, o_cst, o_tst, o_mbar;
+  int o_S, o_V, o_col, o_rcol, o_rrs, o_w2s, o_w2o, o_rag, o_T, o_cst, o_tst, o_mbar;
 };
 
 // ---- PTX helpers -------------------------------------------------------------------
@@ -107,12 +108,6 @@ __device__ __forceinline__ void st_async(uint32_t raddr, cd v, uint32_t rmbar) {
   asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [%0], {%1, %2}, [%3];"
                ::"r"(raddr), "d"(v.x), "d"(v.y), "r"(rmbar) : "memory");
 }
-// bulk copy of this CTA's shared memory into a cluster CTA's, completion counted on its mbarrier
-__device__ __forceinline__ void bulk_push(uint32_t rdst, uint32_t src, uint32_t bytes, uint32_t rmbar) {
-  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(rdst), "r"(src), "r"(bytes), "r"(rmbar) : "memory");
-}
-__device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void mbar_init(uint32_t mbar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar), "r"(count) : "memory");
 }
@@ -315,7 +310,6 @@ __global__ void __launch_bounds__(NT, 1) qr_kernel(QrParams P) {
   cd* Vs = sm + P.o_V;
   cd* colbuf = sm + P.o_col;
   cd* rcol = sm + P.o_rcol;
-  cd* stg = sm + P.o_stg;
   cd* rrs = sm + P.o_rrs;
   cd* w2s = sm + P.o_w2s;
   cd* w2o = sm + P.o_w2o;
@@ -325,7 +319,7 @@ __global__ void __launch_bounds__(NT, 1) qr_kernel(QrParams P) {
   cd* tst = sm + P.o_tst;
   cd* pst = tst + NB * NB;
   uint64_t* mb = reinterpret_cast<uint64_t*>(smem_raw + P.o_mbar);
-  const uint32_t mb_rs = su32(&mb[MB_RS]), mb_ag = su32(&mb[MB_AG]);
+  const uint32_t mb_rs = su32(&mb[MB_RS]), mb_ag = su32(&mb[MB_AG]), rrs32 = su32(rrs), rag32 = su32(rag);
   uint32_t ph_rs = 0, ph_ag = 0;
   bool failed = false;
   cd* Tg = P.T + (int64_t)prob * P.t_b;
@@ -363,7 +357,7 @@ __global__ void __launch_bounds__(NT, 1) qr_kernel(QrParams P) {
     for (int c0 = 0; c0 < ncols; c0 += P.nc) {
       const int ncc = min(P.nc, ncols - c0);
       const int KS = (ncc + C - 1) / C, k0 = crank * KS, ks = max(0, min(ncc, k0 + KS) - k0);
-      const int ntile = (ncc + 7) / 8;
+      const int ntile = (ncc + 7) / 8, inv = (65536 + KS - 1) / KS;   // kk * inv >> 16 == kk / KS for kk < 256
       const bool active = row0 + ROWS > p0;
       if (warp < NWM) {
         // partials over this CTA's rows: 16 x 8 tiles, two per warp in flight
@@ -400,27 +394,24 @@ __global__ void __launch_bounds__(NT, 1) qr_kernel(QrParams P) {
                 }
             }
           }
+          // pushed from the fragments: a store is four runs of eight entries of a column
 #pragma unroll
           for (int u = 0; u < 2; ++u)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const int i = fg + 8 * (e >> 1), kk = 8 * (t + u * NWM) + 2 * ft + (e & 1);
-              if (kk < ncc) stg[kk * LDR + i] = cmk(re[u][e], im[u][e]);
+            for (int c = 0; c < 2; ++c) {
+              const int kk = 8 * (t + u * NWM) + 2 * ft + c;
+              if ((u == 0 || two) && kk < ncc) {
+                const int so = kk * inv >> 16;   // its owner, kk / KS
+                const uint32_t dst = mapa(rrs32, so) + (uint32_t)(((crank * ksc + kk - so * KS) * NB + fg) * sizeof(cd));
+                const uint32_t bar = mapa(mb_rs, so);
+                st_async(dst, cmk(re[u][c], im[u][c]), bar);
+                st_async(dst + 8 * (uint32_t)sizeof(cd), cmk(re[u][2 + c], im[u][2 + c]), bar);
+              }
             }
-        }
-        // each owner's slice of the partials, one bulk copy per rank (16-byte remote stores instead
-        // of these copies took 4 clocks each and set the time of the exchange)
-        fence_async();
-        bar_sync<BAR_TILES, 32 * NWM>();
-        if (warp == 0 && lane < C) {
-          const int q0 = lane * KS, nq = min(ncc, q0 + KS) - q0;
-          if (nq > 0)
-            bulk_push(mapa(su32(&rrs[crank * ksc * LDR]), lane), su32(&stg[q0 * LDR]), (uint32_t)(nq * LDR * sizeof(cd)),
-                      mapa(mb_rs, lane));
         }
       }
       if (ks > 0) {
-        if (tid == 0) mbar_expect(mb_rs, (uint32_t)(C * LDR * ks * sizeof(cd)));
+        if (tid == 0) mbar_expect(mb_rs, (uint32_t)(C * NB * ks * sizeof(cd)));
         cta_wait(mb_rs, ph_rs, failed, err);
         ph_rs ^= 1;
       } else {
@@ -430,10 +421,10 @@ __global__ void __launch_bounds__(NT, 1) qr_kernel(QrParams P) {
       // every CTA; a column's 16 entries sit in one half warp
       for (int e = tid; e < NB * ks; e += NT) {
         const int i = e % NB, kk = e / NB;
-        const cd* src = rrs + kk * LDR + i;
+        const cd* src = rrs + e;
         cd w = cmk(0.0, 0.0);
 #pragma unroll 4
-        for (int q = 0; q < C; ++q) w = cadd(w, src[q * ksc * LDR]);
+        for (int q = 0; q < C; ++q) w = cadd(w, src[q * ksc * NB]);
         w2s[e] = w;
         __syncwarp(__activemask());
         const cd* t = factor ? Ts + LDT * i : Ts + i;
@@ -448,13 +439,15 @@ __global__ void __launch_bounds__(NT, 1) qr_kernel(QrParams P) {
         }
         w2o[kk * LDW + i] = cadd(s0, s1);
       }
-      fence_async();
       __syncthreads();
-      if (warp == 0) {
-        if (lane == 0) mbar_expect(mb_ag, (uint32_t)(ncc * LDW * sizeof(cd)));
-        __syncwarp();
-        if (lane < C && ks > 0)
-          bulk_push(mapa(su32(&rag[k0 * LDW]), lane), su32(w2o), (uint32_t)(ks * LDW * sizeof(cd)), mapa(mb_ag, lane));
+      if (tid == 0) mbar_expect(mb_ag, (uint32_t)(ncc * NB * sizeof(cd)));
+      // a warp takes every eighth rank, two columns per store
+      for (int q = warp; q < C; q += NWM + 1) {
+        const uint32_t dst = mapa(rag32, q), bar = mapa(mb_ag, q);
+        for (int e = lane; e < NB * ks; e += 32) {
+          const int o = (e / NB) * LDW + e % NB;
+          st_async(dst + (uint32_t)((k0 * LDW + o) * sizeof(cd)), w2o[o], bar);
+        }
       }
       cta_wait(mb_ag, ph_ag, failed, err);
       ph_ag ^= 1;
@@ -844,8 +837,7 @@ size_t layout(QrParams& P, int n, int C, int rows, int nc) {
   P.o_V = o;     o += (rows + 1) * NB;
   P.o_col = o;   o += 2 * rows;
   P.o_rcol = o;  o += 2 * (C + 1) * NB;
-  P.o_stg = o;   o += nc * LDR;
-  P.o_rrs = o;   o += C * P.ksc * LDR;
+  P.o_rrs = o;   o += C * P.ksc * NB;
   P.o_w2o = o;   o += P.ksc * LDW;
   P.o_rag = o;   o += nc * LDW;
   P.o_T = o;     o += NB * LDT;
@@ -861,7 +853,9 @@ struct Choice {
 };
 
 // Cluster of C = ceil(m / (32 rpl)) CTAs, at most 16: prefer 1 row per lane, then 2, then 4; the
-// widest column chunk of the block reflectors that fits.  An outer panel of the blocked form
+// widest column chunk of the block reflectors that fits, in steps of 8 (512 x 256, one width against
+// the next: 88 columns 635 us, 64 columns 675, as a chunk costs about 3500 clocks of exchanges
+// whatever its width).  An outer panel of the blocked form
 // (panel) keeps the columns beside an inner panel in one chunk, since its T needs them.
 bool choose(int m, int n, Choice& ch, bool panel = false) {
   QrParams P;
@@ -871,7 +865,7 @@ bool choose(int m, int n, Choice& ch, bool panel = false) {
     const int rows = 32 * rpl;
     const int C = (m + rows - 1) / rows;
     if (C > CMAX) continue;
-    for (int nc = nc_max; nc >= nc_min; nc = nc > 16 ? nc / 16 * 8 : nc - 8) {
+    for (int nc = nc_max; nc >= nc_min; nc -= 8) {
       const size_t b = layout(P, n, C, rows, nc);
       if (b <= SMEM_LIMIT) {
         ch.C = C; ch.rpl = rpl; ch.nc = nc; ch.smem = b;
