@@ -309,58 +309,86 @@ __global__ void oz_split_kernel(SliceView v, const int* __restrict__ rexp0, int6
 // Exponent scan and slicing fused, for operands whose rows fit in shared memory: a CTA holds
 // `rpc` whole rows (all Kc complex columns of the slice grid, zeros beyond K), takes each row's
 // largest exponent and writes its digits -- one read of the operand instead of two and no
-// atomics.  rpc divides 32, so the grid covers the padded rows exactly (rows >= R get exponent
-// 0 and zero digits); exponents and digits are those of the two-pass kernels.
-constexpr int OZ_FUSED_SMEM = 96 * 1024;
+// atomics on memory.  rpc divides 32, so the grid covers the padded rows exactly (rows >= R get
+// exponent 0 and zero digits); exponents and digits are those of the two-pass kernels.
+//
+// Both operands go in one launch, the A' rows' CTAs before the B'^T rows'.  What bounds it is latency
+// and the integer pipe (digits, packing): a thread reads one row, OZ_LOADS elements in flight, with
+// its maximum in a register, and the columns lie 9 apart by 8 in shared memory, so that neither the
+// stores of a column nor the reads of 4 consecutive k conflict.  B200 (cold caches, 6 slices), against
+// one launch per operand with a load in flight and a division per element: 512 x 256 and 256 x 512 in
+// 8 copies 32.5 -> 22.9 us, the larger pairs of these sites 95 -> 52; the slicing of a step of 8
+// trajectories at chi 256 18.8 -> 14.2 ms.  (Rounding by an addition of 1.5 2^52 in place of the
+// conversions to int and back: 14.0, not worth its lines.)
+constexpr int OZ_FUSED_SMEM = 110 * 1024;
+constexpr int OZ_LOADS = 8;
+struct SliceJob {
+  SliceView v;
+  int* rexp; int64_t rexp_bat;
+  int8_t* out; int64_t rows_out;
+  int rpc;         // rows per CTA
+};
+__host__ __device__ constexpr int oz_row_ld(int Kc) { return Kc + Kc / 8 + 1; }
+
 template <int S, bool BMODE>
-__global__ void __launch_bounds__(256)
-    oz_slice_rows_kernel(SliceView v, int* __restrict__ rexp0, int64_t rexp_bat, int8_t* __restrict__ out0,
-                         int64_t rows_out, int Kp, int rpc) {
-  extern __shared__ __align__(16) unsigned char rows_smem[];
-  cd* tile = reinterpret_cast<cd*>(rows_smem);   // [rpc][Kc + 1]
-  __shared__ int rowE[32];
-  const int Kc = Kp / 2, ld = Kc + 1;
-  const int r0 = blockIdx.x * rpc;
-  v.X += (int64_t)blockIdx.z * v.x_bat;
-  int* rexp = rexp0 + (int64_t)blockIdx.z * rexp_bat;
-  int8_t* out = out0 + (int64_t)blockIdx.z * S * rows_out * Kp;
-  const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-  const bool rc = (v.x_r == 1);   // rows contiguous: consecutive threads take consecutive rows
-  const int n = rpc * Kc;
-  for (int e = tid; e < n; e += 256) {
-    int rr, k;
-    if (rc) { rr = e % rpc; k = e / rpc; }
-    else    { k = e % Kc; rr = e / Kc; }
-    const int r = r0 + rr;
-    cd x = cmk(0.0, 0.0);
-    if (r < v.R && k < v.K) {
-      x = v.X[(int64_t)r * v.x_r + (int64_t)k * v.x_k];
-      if (v.conj) x.y = -x.y;
-    }
-    tile[rr * ld + k] = x;
-  }
+__device__ __forceinline__ void slice_rows(const SliceJob& j, int block, int Kp, cd* tile, int* rowE) {
+  const SliceView& v = j.v;
+  const int Kc = Kp / 2, ld = oz_row_ld(Kc), rpc = j.rpc, r0 = block * rpc;
+  const cd* X = v.X + (int64_t)blockIdx.z * v.x_bat;
+  int* rexp = j.rexp + (int64_t)blockIdx.z * j.rexp_bat;
+  int8_t* out = j.out + (int64_t)blockIdx.z * S * j.rows_out * Kp;
+  const int tid = threadIdx.x;
+  if (tid < 32) rowE[tid] = 0;
   __syncthreads();
-  for (int rr = warp; rr < rpc; rr += 8) {
-    int e = 0;
-    for (int k = lane; k < Kc; k += 32) {
-      const cd x = tile[rr * ld + k];
-      e = max(e, (int)((__double_as_longlong(fmax(fabs(x.x), fabs(x.y))) >> 52) & 0x7FF));
+  // consecutive threads along the contiguous index; kt threads of a row
+  const bool rc = (v.x_r == 1);
+  const int kt = 256 / rpc, lkt = 31 - __clz(kt);   // rpc and kt are powers of two
+  const int rr = rc ? (tid & (rpc - 1)) : tid >> lkt, kf = rc ? tid / rpc : (tid & (kt - 1));
+  const int r = r0 + rr;
+  const cd* src = X + (int64_t)r * v.x_r;
+  int em = 0;
+  for (int k0 = kf; k0 < Kc; k0 += OZ_LOADS * kt) {
+    cd x[OZ_LOADS];
+#pragma unroll
+    for (int q = 0; q < OZ_LOADS; ++q) {
+      const int k = k0 + q * kt;
+      x[q] = cmk(0.0, 0.0);
+      if (r < v.R && k < v.K) x[q] = src[(int64_t)k * v.x_k];
     }
-    for (int o = 16; o; o >>= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
-    if (lane == 0) {
-      rowE[rr] = e;
-      if (r0 + rr < v.R) rexp[r0 + rr] = e;
+#pragma unroll
+    for (int q = 0; q < OZ_LOADS; ++q) {
+      const int k = k0 + q * kt;
+      if (k >= Kc) break;
+      if (v.conj) x[q].y = -x[q].y;
+      em = max(em, (int)((__double_as_longlong(fmax(fabs(x[q].x), fabs(x[q].y))) >> 52) & 0x7FF));
+      tile[rr * ld + k + (k >> 3)] = x[q];
     }
   }
+  if (em > 0) atomicMax(&rowE[rr], em);
   __syncthreads();
+  if (tid < rpc && r0 + tid < v.R) rexp[r0 + tid] = rowE[tid];
   const int q4 = Kc / 4;   // items of 4 complex k per row
-  for (int it = tid; it < rpc * q4; it += 256) {
-    const int rr = it / q4, kq = (it % q4) * 4;
-    const int r = r0 + rr;
-    const cd* tp = tile + rr * ld + kq;
+  int ir = tid / q4, ik = tid - ir * q4;   // this item's row and place; the next is 256 items on
+  const int dr = 256 / q4, dk = 256 - dr * q4;
+  while (ir < rpc) {
+    const int ri = r0 + ir, kq = 4 * ik;
+    const cd* tp = tile + ir * ld + kq + (kq >> 3);
     const cd xs[4] = {tp[0], tp[1], tp[2], tp[3]};
-    store_digits<S, BMODE>(out, rows_out, Kp, r, 2 * (int64_t)kq, xs, row_scale(r < v.R ? rowE[rr] : 0));
+    store_digits<S, BMODE>(out, j.rows_out, Kp, ri, 2 * (int64_t)kq, xs, row_scale(ri < v.R ? rowE[ir] : 0));
+    ir += dr;
+    ik += dk;
+    if (ik >= q4) { ik -= q4; ++ir; }
   }
+}
+
+template <int S>
+__global__ void __launch_bounds__(256)
+    oz_slice_rows_kernel(const __grid_constant__ SliceJob a, const __grid_constant__ SliceJob b, int na, int Kp) {
+  extern __shared__ __align__(16) unsigned char rows_smem[];
+  __shared__ int rowE[32];
+  cd* tile = reinterpret_cast<cd*>(rows_smem);   // [rpc][oz_row_ld(Kc)]
+  if ((int)blockIdx.x < na) slice_rows<S, false>(a, blockIdx.x, Kp, tile, rowE);
+  else slice_rows<S, true>(b, blockIdx.x - na, Kp, tile, rowE);
 }
 
 // ---------------------------------------------------------------- the tensor-core GEMM
@@ -640,13 +668,13 @@ int device_sm_count() {
 
 typedef void (*OzKernel)(CUtensorMap, CUtensorMap, OzParams);
 typedef void (*SplitKernel)(SliceView, const int*, int64_t, int8_t*, int64_t, int);
-typedef void (*FusedKernel)(SliceView, int*, int64_t, int8_t*, int64_t, int, int);
+typedef void (*FusedKernel)(SliceJob, SliceJob, int, int);
 
 template <int S>
 struct OzTable {
   static OzKernel gemm() { return ozgemm_kernel<S>; }
   static SplitKernel split(bool b) { return b ? oz_split_kernel<S, true> : oz_split_kernel<S, false>; }
-  static FusedKernel fused(bool b) { return b ? oz_slice_rows_kernel<S, true> : oz_slice_rows_kernel<S, false>; }
+  static FusedKernel fused() { return oz_slice_rows_kernel<S>; }
   static int smem() { return smem_bytes(S); }
 };
 
@@ -670,13 +698,13 @@ SplitKernel pick_split(int S, bool b) {
   }
   return nullptr;
 }
-FusedKernel pick_fused(int S, bool b) {
+FusedKernel pick_fused(int S) {
   switch (S) {
-    case 3: return OzTable<3>::fused(b);
-    case 4: return OzTable<4>::fused(b);
-    case 5: return OzTable<5>::fused(b);
-    case 6: return OzTable<6>::fused(b);
-    case 7: return OzTable<7>::fused(b);
+    case 3: return OzTable<3>::fused();
+    case 4: return OzTable<4>::fused();
+    case 5: return OzTable<5>::fused();
+    case 6: return OzTable<6>::fused();
+    case 7: return OzTable<7>::fused();
   }
   return nullptr;
 }
@@ -745,7 +773,7 @@ int ozgemm_launch(const Gemm& g, int slices, void* scratch, size_t scratch_bytes
   auto fused_rows = [&](const SliceView& v, int64_t rows_padded) {
     const int floor_rows = (v.x_r == 1) ? 8 : 1;
     int rpc = 32;
-    while (rpc >= floor_rows && (size_t)rpc * (kc + 1) * sizeof(cd) > (size_t)OZ_FUSED_SMEM) rpc /= 2;
+    while (rpc >= floor_rows && (size_t)rpc * oz_row_ld(kc) * sizeof(cd) > (size_t)OZ_FUSED_SMEM) rpc /= 2;
     if (rpc < floor_rows) return 0;
     while (rpc > floor_rows && rows_padded * B / rpc < 2 * 148) rpc /= 2;
     return rpc;
@@ -760,29 +788,30 @@ int ozgemm_launch(const Gemm& g, int slices, void* scratch, size_t scratch_bytes
     const int64_t tiles = (int64_t)((rows + 31) / 32) * ktiles * B;
     return (int)std::max<int64_t>(1, std::min<int64_t>(8, tiles / (148 * 8)));
   };
-  auto slice = [&](const SliceView& v, int* e, int64_t rows_padded, int8_t* dst, int64_t rows_out, bool bmode,
-                   int rpc) -> int {
+  auto two_pass = [&](const SliceJob& j, int64_t rows_padded, bool bmode) -> int {
+    const int kp = kper(j.v.R);
     count_launch(ws);
-    if (rpc > 0) {
-      FusedKernel fk = pick_fused(S, bmode);
-      const int smem = (int)((size_t)rpc * (kc + 1) * sizeof(cd));
-      MPSB_TRY(ensure_kernel_attrs((const void*)fk, OZ_FUSED_SMEM));
-      fk<<<dim3((unsigned)(rows_padded / rpc), 1, bz), 256, smem, s>>>(v, e, rows_padded, dst, rows_out, (int)Kp, rpc);
-      MPSB_CUDA_TRY(cudaGetLastError());
-      return MPSB_OK;
-    }
-    const int kp = kper(v.R);
-    oz_rowexp_kernel<<<dim3((unsigned)((v.R + 31) / 32), (unsigned)((ktiles + kp - 1) / kp), bz), 256, 0, s>>>(
-        v, e, rows_padded, kp);
+    oz_rowexp_kernel<<<dim3((unsigned)((j.v.R + 31) / 32), (unsigned)((ktiles + kp - 1) / kp), bz), 256, 0, s>>>(
+        j.v, j.rexp, j.rexp_bat, kp);
     MPSB_CUDA_TRY(cudaGetLastError());
     count_launch(ws);
     pick_split(S, bmode)<<<dim3((unsigned)(rows_padded / 32), (unsigned)(kc / 32), bz), 256, 0, s>>>(
-        v, e, rows_padded, dst, rows_out, (int)Kp);
+        j.v, j.rexp, j.rexp_bat, j.out, j.rows_out, (int)Kp);
     MPSB_CUDA_TRY(cudaGetLastError());
     return MPSB_OK;
   };
-  MPSB_TRY(slice(va, ea, Mpad, sa, Mpad, false, ra));
-  MPSB_TRY(slice(vb, eb, NBpad / 2, sb, NBpad, true, rb));
+  const SliceJob ja{va, ea, Mpad, sa, Mpad, ra}, jb{vb, eb, NBpad / 2, sb, NBpad, rb};
+  if (ra == 0) MPSB_TRY(two_pass(ja, Mpad, false));
+  if (rb == 0) MPSB_TRY(two_pass(jb, NBpad / 2, true));
+  const int64_t na = ra > 0 ? Mpad / ra : 0, nb = rb > 0 ? NBpad / 2 / rb : 0;
+  if (na + nb > 0) {
+    FusedKernel fk = pick_fused(S);
+    MPSB_TRY(ensure_kernel_attrs((const void*)fk, OZ_FUSED_SMEM));
+    count_launch(ws);
+    fk<<<dim3((unsigned)(na + nb), 1, bz), 256, (size_t)std::max(ra, rb) * oz_row_ld(kc) * sizeof(cd), s>>>(
+        ja, jb, (int)na, (int)Kp);
+    MPSB_CUDA_TRY(cudaGetLastError());
+  }
 
   CUtensorMap ta, tb;
   MPSB_TRY(make_map(&ta, sa, Kp, B * S * Mpad, OZ_BM));
