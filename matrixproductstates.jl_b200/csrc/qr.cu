@@ -48,13 +48,14 @@
 // Shapes beyond one cluster (for example 2048 x 512) are factored in outer panels of up to 64
 // columns by the same kernel, with the trailing updates and Q as GEMMs (qr_blocked).
 //
-// What bounds it: the chain of column steps (512 x 128: 2350 clocks a step at 16 CTAs, 60 % of the
-// time, 4-6 clocks an instruction; 2140 at 4 CTAs, 1340 at one), then the products, which run at the
-// FP64 tensor rate of the cluster's SMs.  One row per lane and many CTAs beat more rows per lane
-// (512 x 128 at 1 / 2 / 4 rows: 254 / 324 / 491 us) because the products scale with the CTAs.
+// What bounds it: the chain of column steps (512 x 128: 2260 clocks a step at 16 CTAs -- sums over the
+// rows 600, exchange 730, sum over the ranks 330, reflector 380, update 270 -- 55 % of the time; fewer
+// at fewer CTAs, 1300 at one), then the products, which run at the FP64 tensor rate of the cluster's
+// SMs.  One row per lane and many CTAs beat more rows per lane (512 x 128 at 1 / 2 / 4 rows: 254 / 324
+// / 491 us) because the products scale with the CTAs.
 // Against the form with a reflector warp behind block barriers, Q as GEMMs over a back substitution
-// and outer panels of 16 columns (B200, Q only): 64 x 32 108.7 -> 50.2 us, 512 x 128 394 -> 248,
-// 512 x 256 818 -> 635, 2048 x 512 3990 -> 2140.
+// and outer panels of 16 columns (B200, Q only): 64 x 32 108.7 -> 49.7 us, 512 x 128 394 -> 238,
+// 512 x 256 818 -> 598, 2048 x 512 3990 -> 2080.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -91,7 +92,7 @@ struct QrParams {
   int64_t t_ld, t_b;
   int C, npanels, ldS, nc, ksc;   // nc: columns per exchange of a block reflector, ksc = ceil(nc / C)
   // shared-memory offsets (complex elements) and the byte offset of the mbarriers
-  int o_S, o_V, o_col, o_rcol, o_rrs, o_w2s, o_w2o, o_rag, o_T, o_cst, o_tst, o_mbar;
+  int o_S, o_V, o_col, o_rcol, o_rrs, o_w2s, o_rag, o_T, o_cst, o_tst, o_mbar;
 };
 
 // ---- PTX helpers -------------------------------------------------------------------
@@ -189,7 +190,7 @@ __device__ __forceinline__ int scale_of_nan(double v) { return (int)((__double_a
 // every lane tau, beta, rs = 1/(alpha - beta) at 2^-E, and fE = 2^-E.  Returned by value, so
 // the caller's variables stay in registers on the common path.
 struct Reflector {
-  cd s, tau, rs, xj;
+  cd s, tau, rs;
   double beta_x, beta_y, ib, fE;
 };
 __device__ __noinline__ Reflector reflector_scaled(const cd* rb, int C, int lane, int jl, int pw, cd alpha) {
@@ -220,7 +221,7 @@ __device__ __noinline__ Reflector reflector_scaled(const cd* rb, int C, int lane
   const unsigned ha = (unsigned)__double2hiint(fmax(fabs(alpha.x), fabs(alpha.y)));
   o.fE = 1.0;
   o.s = v;
-  o.tau = cmk(0.0, 0.0); o.rs = cmk(1.0, 0.0); o.xj = cmk(0.0, 0.0); o.ib = 0.0;
+  o.tau = cmk(0.0, 0.0); o.rs = cmk(1.0, 0.0); o.ib = 0.0;
   o.beta_x = alpha.x; o.beta_y = alpha.y;
   if (ex == ESENT && (alpha.y == 0.0 || ha == 0u)) return o;   // x == 0 and a real (or negligible) pivot: H = I
   int ea = expo_hi(ha);
@@ -238,7 +239,6 @@ __device__ __noinline__ Reflector reflector_scaled(const cd* rb, int C, int lane
   o.beta_x = b * pow2i(E);
   o.beta_y = 0.0;
   o.rs = cmk(dr * id, -as.y * id);
-  o.xj = cmk(dr, as.y);
   o.s = (ex == ESENT) ? cmk(0.0, 0.0) : cscal(v, pow2neg(ex - E));
   return o;
 }
@@ -262,7 +262,7 @@ __device__ __forceinline__ double rcp_seed(double a) {
 // alpha lie inside the window -- tested on the high words, beside the formula: 0 < xn2 < 2^1023 and
 // |Re alpha|, |Im alpha| < 2^SWIN; returns false otherwise.
 //   tau = (beta - alpha)/beta, rs = 1/(alpha - beta) = conj(alpha - beta)/|alpha - beta|^2 with
-//   |alpha - beta|^2 = |alpha|^2 + beta^2 + 2 |Re alpha| |beta|, xj = alpha - beta, ib = 1/beta
+//   |alpha - beta|^2 = |alpha|^2 + beta^2 + 2 |Re alpha| |beta|, ib = 1/beta
 // (beta carries the opposite sign of Re alpha, so nothing cancels).  It sits on the critical path of
 // every column, so |beta| = sqrt(n2), 1/|beta| and the reciprocal come from the hardware's 20-bit
 // seeds, the second taken from the first's unrefined value, and one third-order Newton-Raphson
@@ -283,8 +283,7 @@ __device__ __forceinline__ bool reflector(cd alpha, double xn2, Reflector& o) {
   o.beta_x = -copysign(nrm, alpha.x);
   o.beta_y = 0.0;
   o.tau = cmk(fma(-alpha.x, o.ib, 1.0), -alpha.y * o.ib);
-  o.xj = cmk(alpha.x - o.beta_x, alpha.y);
-  o.rs = cmk(o.xj.x * z, -alpha.y * z);
+  o.rs = cmk((alpha.x - o.beta_x) * z, -alpha.y * z);
   return in;
 }
 // a - f v
@@ -312,7 +311,6 @@ __global__ void __launch_bounds__(NT, 1) qr_kernel(QrParams P) {
   cd* rcol = sm + P.o_rcol;
   cd* rrs = sm + P.o_rrs;
   cd* w2s = sm + P.o_w2s;
-  cd* w2o = sm + P.o_w2o;
   cd* rag = sm + P.o_rag;
   cd* Ts = sm + P.o_T;
   cd* cst = sm + P.o_cst;
@@ -417,37 +415,41 @@ __global__ void __launch_bounds__(NT, 1) qr_kernel(QrParams P) {
       } else {
         __syncthreads();
       }
-      // the ranks' sum and op(T) W on my slice (zero beyond the panel width: V and T are), copied to
-      // every CTA; a column's 16 entries sit in one half warp
-      for (int e = tid; e < NB * ks; e += NT) {
-        const int i = e % NB, kk = e / NB;
-        const cd* src = rrs + e;
-        cd w = cmk(0.0, 0.0);
-#pragma unroll 4
-        for (int q = 0; q < C; ++q) w = cadd(w, src[q * ksc * NB]);
-        w2s[e] = w;
-        __syncwarp(__activemask());
-        const cd* t = factor ? Ts + LDT * i : Ts + i;
+      // the ranks' sum and op(T) W on my slice (zero beyond the panel width: V and T are), a warp per
+      // column: a lane has entry i, half of the ranks, half of the products and half of the pushes
+      if (tid == 0) mbar_expect(mb_ag, (uint32_t)(ncc * NB * sizeof(cd)));
+      for (int kk = warp; kk < ks; kk += NWM + 1) {
+        const int i = lane & 15, h = lane >> 4;
+        const cd* src = rrs + kk * NB + i;
+        const int rs = ksc * NB;
+        cd w = cmk(0.0, 0.0), w1 = cmk(0.0, 0.0);
+#pragma unroll 2
+        for (int q = h; q < C; q += 4) {
+          w = cadd(w, src[q * rs]);
+          if (q + 2 < C) w1 = cadd(w1, src[(q + 2) * rs]);
+        }
+        w = cadd(w, w1);
+        w.x += __shfl_xor_sync(0xffffffffu, w.x, 16);
+        w.y += __shfl_xor_sync(0xffffffffu, w.y, 16);
+        cd* wc = w2s + kk * NB;
+        if (h == 0) wc[i] = w;
+        __syncwarp();
+        const cd* t = (factor ? Ts + LDT * i : Ts + i);
         const int ts = factor ? 1 : LDT;
         cd s0 = cmk(0.0, 0.0), s1 = cmk(0.0, 0.0);
-#pragma unroll 4
-        for (int i2 = 0; i2 < NB; i2 += 2) {
+#pragma unroll
+        for (int i2 = 8 * h; i2 < 8 * h + 8; i2 += 2) {
           cd t0 = t[i2 * ts], t1 = t[(i2 + 1) * ts];
           if (factor) { t0.y = -t0.y; t1.y = -t1.y; }
-          cfma(s0, t0, w2s[kk * NB + i2]);
-          cfma(s1, t1, w2s[kk * NB + i2 + 1]);
+          cfma(s0, t0, wc[i2]);
+          cfma(s1, t1, wc[i2 + 1]);
         }
-        w2o[kk * LDW + i] = cadd(s0, s1);
-      }
-      __syncthreads();
-      if (tid == 0) mbar_expect(mb_ag, (uint32_t)(ncc * NB * sizeof(cd)));
-      // a warp takes every eighth rank, two columns per store
-      for (int q = warp; q < C; q += NWM + 1) {
-        const uint32_t dst = mapa(rag32, q), bar = mapa(mb_ag, q);
-        for (int e = lane; e < NB * ks; e += 32) {
-          const int o = (e / NB) * LDW + e % NB;
-          st_async(dst + (uint32_t)((k0 * LDW + o) * sizeof(cd)), w2o[o], bar);
-        }
+        s0 = cadd(s0, s1);
+        s0.x += __shfl_xor_sync(0xffffffffu, s0.x, 16);
+        s0.y += __shfl_xor_sync(0xffffffffu, s0.y, 16);
+        const uint32_t off = (uint32_t)(((k0 + kk) * LDW + i) * sizeof(cd));
+#pragma unroll 2
+        for (int q = h; q < C; q += 2) st_async(mapa(rag32, q) + off, s0, mapa(mb_ag, q));
       }
       cta_wait(mb_ag, ph_ag, failed, err);
       ph_ag ^= 1;
@@ -556,6 +558,12 @@ __global__ void __launch_bounds__(NT, 1) qr_kernel(QrParams P) {
           if (warp == 0) mbar_expect(mbc, (uint32_t)((C + 1) * NB * sizeof(cd)));
           else mbar_arrive(mbc);
         }
+        const uint32_t ob = (uint32_t)(buf * rbuf * sizeof(cd)), om = 8 * buf;
+        if (!SOLO && owner) {   // the pivot row is known before the sums: its flight is hidden
+          const cd piv = cs[NB + pc];
+          if (push0) st_async(rd0 + ob + off_piv, piv, rm0 + om);
+          if (push1) st_async(rd1 + ob + off_piv, piv, rm1 + om);
+        }
         // -- partial sums of conj(x) a over this CTA's rows g > j (x zero elsewhere)
 #pragma unroll
         for (int q = 0; q < RPL; ++q)
@@ -617,19 +625,14 @@ __global__ void __launch_bounds__(NT, 1) qr_kernel(QrParams P) {
         // this warp's columns, the pivot and the next; for one warp all, for T
         const bool keeps = warp == (((jl >> 2) + 2) & 3), need = keeps || (c >> 2) == warp || c == jl || c == jl + 1;
         const cd* rb = SOLO ? cs : rcol + buf * rbuf;
+        const cd* pv = SOLO ? cs + NB : rb + C * NB;   // the pivot row's entries
         cd rv, s;
         if (!SOLO) {
-          const uint32_t ob = (uint32_t)(buf * rbuf * sizeof(cd)), om = 8 * buf;
           if (push0) st_async(rd0 + ob + off_sum, sum, rm0 + om);
           if (push1) st_async(rd1 + ob + off_sum, sum, rm1 + om);
-          if (owner) {
-            const cd piv = cs[NB + pc];
-            if (push0) st_async(rd0 + ob + off_piv, piv, rm0 + om);
-            if (push1) st_async(rd1 + ob + off_piv, piv, rm1 + om);
-          }
           warp_wait(mbc, (uint32_t)(step >> 1) & 1, failed, err);
           const int h = (lane >> 4) * 8;   // lane c sums ranks 0 .. 7 of column c, lane c + 16 the others
-          rv = rb[C * NB + c];
+          rv = pv[c];
           cd part[8];
 #pragma unroll
           for (int q = 0; q < 8; ++q) part[q] = need && h + q < C ? rb[(h + q) * NB + c] : cmk(0.0, 0.0);
@@ -644,19 +647,38 @@ __global__ void __launch_bounds__(NT, 1) qr_kernel(QrParams P) {
           if (pr == 0) cs[pc] = sum;
           bar_sync<BAR_PANEL, 32 * (NWP + 1)>();
           s = cs[c];
-          rv = cs[NB + c];
+          rv = pv[c];
         }
         // -- the reflector, formed by every warp from the same sums
         cd nx[RPL];   // column jl + 1 as updated by the reflectors before this one
 #pragma unroll
         for (int q = 0; q < RPL; ++q) nx[q] = colbuf[((jl + 1) & 1) * ROWS + lane + 32 * q];
-        const cd alpha = shfl(rv, jl);
+        // this warp's columns' sums and pivot entries, and the next column's, in every lane: read
+        // back from shared memory while the reflector's chain runs (4 rows per lane: after it, as the
+        // registers do not suffice)
+        cd* sb = rag + NB * warp;
+        if (lane < NB) sb[lane] = s;
+        __syncwarp();
+        const int jn = min(jl + 1, NB - 1);
+        cd sk[CW], rk[CW], sn, rn;
+        auto fetch = [&] {
+          sn = sb[jn];
+          rn = pv[jn];
+#pragma unroll
+          for (int k = 0; k < CW; ++k) { sk[k] = sb[cf + k]; rk[k] = pv[cf + k]; }
+        };
+        if (RPL < 4) fetch();
+        const cd alpha = pv[jl];
         const double xn2 = __shfl_sync(0xffffffffu, s.x, jl);
         Reflector o;
         const bool plain = reflector(alpha, xn2, o);
         if (__builtin_expect(!plain, 0)) {
           o = reflector_scaled(rb, C, c, jl, pw, alpha);
           s = o.s;
+          __syncwarp();
+          if (lane < NB) sb[lane] = s;
+          __syncwarp();
+          if (RPL < 4) fetch();
 #pragma unroll
           for (int q = 0; q < RPL; ++q) {   // v = rs x 2^-E; column j is kept as v itself
             x[q] = cscal(x[q], o.fE);
@@ -665,21 +687,23 @@ __global__ void __launch_bounds__(NT, 1) qr_kernel(QrParams P) {
               if (cf + k == jl && row0 + lane + 32 * q > j) a[k][q] = cmul(o.rs, x[q]);
           }
         }
-        // lane c right of the pivot: a_c -= f v with f = conj(tau) (a_c[j] + conj(rs) x^H a_c) =
-        // conj(tau) a_c[j] - (x^H a_c)/beta and v = rs x, 1 at the pivot where x is set to 1/rs
-        const cd f = cmk(fma(o.tau.x, rv.x, fma(o.tau.y, rv.y, -o.ib * s.x)), fma(o.tau.x, rv.y, fma(-o.tau.y, rv.x, -o.ib * s.y)));
-        const cd hh = c > jl ? cmul(f, o.rs) : cmk(0.0, 0.0);
-        const cd hn = shfl(hh, min(jl + 1, NB - 1));
-        cd hk[CW];
-#pragma unroll
-        for (int k = 0; k < CW; ++k) hk[k] = shfl(hh, cf + k);
+        // right of the pivot: a_c -= f_c v with f_c = conj(tau) (a_c[j] + conj(rs) x^H a_c) =
+        // conj(tau) a_c[j] - (x^H a_c)/beta and v = rs x, 1 at the pivot
+        auto factor = [&](cd r, cd t) {
+          return cmk(fma(o.tau.x, r.x, fma(o.tau.y, r.y, -o.ib * t.x)), fma(o.tau.x, r.y, fma(-o.tau.y, r.x, -o.ib * t.y)));
+        };
         if (o.tau.x != 0.0 || o.tau.y != 0.0) {   // else H = I
+          if (RPL == 4) fetch();
+          const cd fn = factor(rn, sn);
+          cd fk[CW];
+#pragma unroll
+          for (int k = 0; k < CW; ++k) fk[k] = cf + k > jl ? factor(rk[k], sk[k]) : cmk(0.0, 0.0);
 #pragma unroll
           for (int q = 0; q < RPL; ++q) {
-            if (row0 + lane + 32 * q == j) x[q] = o.xj;
+            const cd v = row0 + lane + 32 * q == j ? cmk(1.0, 0.0) : cmul(o.rs, x[q]);
+            x[q] = cfms(nx[q], fn, v);
 #pragma unroll
-            for (int k = 0; k < CW; ++k) a[k][q] = cfms(a[k][q], hk[k], x[q]);
-            x[q] = cfms(nx[q], hn, x[q]);
+            for (int k = 0; k < CW; ++k) a[k][q] = cfms(a[k][q], fk[k], v);
           }
         } else {
 #pragma unroll
@@ -838,7 +862,6 @@ size_t layout(QrParams& P, int n, int C, int rows, int nc) {
   P.o_col = o;   o += 2 * rows;
   P.o_rcol = o;  o += 2 * (C + 1) * NB;
   P.o_rrs = o;   o += C * P.ksc * NB;
-  P.o_w2o = o;   o += P.ksc * LDW;
   P.o_rag = o;   o += nc * LDW;
   P.o_T = o;     o += NB * LDT;
   P.o_cst = P.o_w2s = o;   o += std::max(4, P.ksc) * NB;   // column steps / block reflectors
