@@ -54,8 +54,8 @@
 // SMs.  One row per lane and many CTAs beat more rows per lane (512 x 128 at 1 / 2 / 4 rows: 254 / 324
 // / 491 us) because the products scale with the CTAs.
 // Against the form with a reflector warp behind block barriers, Q as GEMMs over a back substitution
-// and outer panels of 16 columns (B200, Q only): 64 x 32 108.7 -> 49.7 us, 512 x 128 394 -> 238,
-// 512 x 256 818 -> 598, 2048 x 512 3990 -> 2080.
+// and outer panels of 16 columns (B200, Q only): 64 x 32 108.7 -> 47.6 us, 512 x 128 394 -> 235,
+// 512 x 256 818 -> 590, 2048 x 512 3990 -> 2090.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -79,6 +79,11 @@ constexpr int WAIT_LIMIT = 1 << 20;
 constexpr int LDT = NB + 1, LDW = NB + 1;   // leading dimensions of T, the gathered W
 enum { MB_COL = 0, MB_RS = 2, MB_AG, MB_COUNT };
 constexpr int BAR_PANEL = 1, BAR_END = 2;   // named barriers: a step (C == 1), a panel's end
+
+// Slots of the ranks' partial sums in a column's exchange: a power of two, the unused ones zero, so
+// that a lane's sum over its half needs no tests (against sums tested per rank and column: 64 x 32
+// 49.7 -> 47.6 us, 162 x 81 145.9 -> 142.0, 512 x 128 237.9 -> 235.1).
+__host__ __device__ constexpr int rank_slots(int C) { return C <= 2 ? 2 : (C <= 4 ? 4 : (C <= 8 ? 8 : 16)); }
 
 struct QrParams {
   QrProblem p;
@@ -309,6 +314,7 @@ __global__ void __launch_bounds__(NT, 1) qr_kernel(QrParams P) {
   cd* Vs = sm + P.o_V;
   cd* colbuf = sm + P.o_col;
   cd* rcol = sm + P.o_rcol;
+  const int CP = rank_slots(C), rbuf = (CP + 1) * NB;
   cd* rrs = sm + P.o_rrs;
   cd* w2s = sm + P.o_w2s;
   cd* rag = sm + P.o_rag;
@@ -344,6 +350,7 @@ __global__ void __launch_bounds__(NT, 1) qr_kernel(QrParams P) {
     if (!P.form_q && crank == 0)
       for (int e = tid; e < n * n; e += NT) Tg[(e % n) + (int64_t)(e / n) * P.t_ld] = cmk(0.0, 0.0);
   }
+  for (int e = tid; e < 2 * rbuf; e += NT) rcol[e] = cmk(0.0, 0.0);   // the slots of ranks >= C stay zero
   cluster.sync();   // mbarriers initialised cluster-wide before any push
 
   // Columns kk in [0, ncols) -- columns 0 .. nprev-1 of the matrix, then cbase, cbase + 1, ... --
@@ -515,7 +522,6 @@ __global__ void __launch_bounds__(NT, 1) qr_kernel(QrParams P) {
   // Two buffers of the exchange suffice: another CTA pushes step j + 2 after its exchange of step
   // j + 1, so after every panel warp here pushed step j + 1, which each does when it has read step j.
   int step = 0;   // column steps so far: buffers step & 1, phase parity (step / 2) & 1
-  const int rbuf = (C + 1) * NB;
   const int pr = lane & 7, pc = CW * warp + (lane >> 3);   // this lane pushes column pc to ranks pr, pr + 8
   const bool push0 = pr < C, push1 = pr + 8 < C;
   uint32_t rd0, rd1, rm0, rm1;   // where: slot pc of this rank's row, and the exchange's mbarriers
@@ -524,7 +530,7 @@ __global__ void __launch_bounds__(NT, 1) qr_kernel(QrParams P) {
     rd0 = mapa(slot, push0 ? pr : 0); rm0 = mapa(m0, push0 ? pr : 0);
     rd1 = mapa(slot, push1 ? pr + 8 : 0); rm1 = mapa(m0, push1 ? pr + 8 : 0);
   }
-  const uint32_t off_sum = (uint32_t)(crank * NB * sizeof(cd)), off_piv = (uint32_t)(C * NB * sizeof(cd));
+  const uint32_t off_sum = (uint32_t)(crank * NB * sizeof(cd)), off_piv = (uint32_t)(CP * NB * sizeof(cd));
   if (warp == NWM && lane == 0)   // the T warp's arrivals for the first two steps
     for (int k = 0; k < 2; ++k) mbar_arrive(su32(&mb[MB_COL + k]));
   for (int pi = 0; pi < P.npanels; ++pi) {
@@ -622,25 +628,28 @@ __global__ void __launch_bounds__(NT, 1) qr_kernel(QrParams P) {
         if (scaled && pc == jl) sum = cmk(scale_nan(expo_hi(hb)), sum.x);
         // -- the exchange: every CTA gets all ranks' sums and the pivot row
         const int c = lane & 15;
-        // this warp's columns, the pivot and the next; for one warp all, for T
-        const bool keeps = warp == (((jl >> 2) + 2) & 3), need = keeps || (c >> 2) == warp || c == jl || c == jl + 1;
+        const bool keeps = warp == (((jl >> 2) + 2) & 3);   // writes what T needs
         const cd* rb = SOLO ? cs : rcol + buf * rbuf;
-        const cd* pv = SOLO ? cs + NB : rb + C * NB;   // the pivot row's entries
+        const cd* pv = SOLO ? cs + NB : rb + CP * NB;   // the pivot row's entries
         cd rv, s;
         if (!SOLO) {
           if (push0) st_async(rd0 + ob + off_sum, sum, rm0 + om);
           if (push1) st_async(rd1 + ob + off_sum, sum, rm1 + om);
           warp_wait(mbc, (uint32_t)(step >> 1) & 1, failed, err);
-          const int h = (lane >> 4) * 8;   // lane c sums ranks 0 .. 7 of column c, lane c + 16 the others
+          // lane c sums one half of the slots of column c, lane c + 16 the other
+          const cd* rp = rb + (lane >> 4) * (CP / 2) * NB + c;
           rv = pv[c];
-          cd part[8];
+          s = rp[0];
+          if (CP == 16) {
+            cd p[8];
 #pragma unroll
-          for (int q = 0; q < 8; ++q) part[q] = need && h + q < C ? rb[(h + q) * NB + c] : cmk(0.0, 0.0);
-#pragma unroll
-          for (int w = 4; w > 0; w >>= 1)
-#pragma unroll
-            for (int q = 0; q < w; ++q) part[q] = cadd(part[q], part[q + w]);
-          s = part[0];
+            for (int q = 0; q < 8; ++q) p[q] = rp[q * NB];
+            s = cadd(cadd(cadd(p[0], p[4]), cadd(p[2], p[6])), cadd(cadd(p[1], p[5]), cadd(p[3], p[7])));
+          } else if (CP == 8) {
+            s = cadd(cadd(s, rp[2 * NB]), cadd(rp[NB], rp[3 * NB]));
+          } else if (CP == 4) {
+            s = cadd(s, rp[NB]);
+          }
           s.x += __shfl_xor_sync(0xffffffffu, s.x, 16);
           s.y += __shfl_xor_sync(0xffffffffu, s.y, 16);
         } else {
@@ -860,7 +869,7 @@ size_t layout(QrParams& P, int n, int C, int rows, int nc) {
   P.o_S = o;     o += P.ldS * n;
   P.o_V = o;     o += (rows + 1) * NB;
   P.o_col = o;   o += 2 * rows;
-  P.o_rcol = o;  o += 2 * (C + 1) * NB;
+  P.o_rcol = o;  o += 2 * (rank_slots(C) + 1) * NB;
   P.o_rrs = o;   o += C * P.ksc * NB;
   P.o_rag = o;   o += nc * LDW;
   P.o_T = o;     o += NB * LDT;
