@@ -15,7 +15,7 @@ struct mpsb_ctx {
   cudaStream_t stream = nullptr;
   mpsb::Workspace ws;
   // second lane of the RK4 step: the next stage's environment initialisation runs on `side`
-  // with its own scratch and split-K workspace (swapped into `ws`/`stream` while it issues)
+  // with its own scratch (swapped into `ws`/`stream` while it issues)
   cudaStream_t side = nullptr;
   mpsb::Workspace ws_side;
   std::vector<cudaEvent_t> events;   // per-site / fork / join events, created on first use
