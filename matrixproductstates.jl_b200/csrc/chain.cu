@@ -7,13 +7,14 @@
 // Site k is a matrix-vector product with u = v (x) f over rows r = (a, s), the fastest index of B_k, so
 // a CTA's slice of columns b is one contiguous block of the slab.  Those blocks do not depend on v:
 // thread 0 streams the CTA's blocks of all sites through a ring of bulk copies, sites ahead of the
-// arithmetic.  A warp's lanes take a column's rows (up to eight warps share a column when a ring slot
-// holds few), the CTA's part of v' goes to every CTA by remote stores, and one cluster barrier ends
-// the site.
+// arithmetic.  A warp takes a column and pushes its entry of v' to every CTA with st.async, counted on
+// the receiver's mbarrier, which is the site's only synchronisation between CTAs; sites whose blocks
+// take more than half of the ring go slot by slot (up to eight warps share a column there).
 //
-// What bounds it: a site's chain u -> sums -> remote stores -> cluster barrier, about 3 us; the 1 MB of
-// a chi = 128, d = 4 site passes underneath.  40 sites at chi = 128, d = 4, read-back included: 143 us
-// against 495 us for two GEMM launches per site (M or N = 1).
+// What bounds it: a site's chain u -> sums -> exchange, about 2.2 us; the 1 MB of a chi = 128, d = 4 site
+// passes underneath.  40 sites at chi = 128, d = 4, read-back included: 105 us, against 143 with a
+// cluster barrier per site and the slots one by one, and 495 for two GEMM launches per site (M or
+// N = 1).
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -46,10 +47,32 @@ struct Smem {
   cd v[2][CHI];
   cd f[FUN];
   cd part[CHI / C][NW];
-  uint64_t full[NSLOT];
+  uint64_t full[NSLOT], vfull[2];
 };
 
 __device__ __forceinline__ uint32_t su32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
+
+__device__ __forceinline__ uint32_t mapa(uint32_t a, int rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void expect(uint64_t* m, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(su32(m)), "r"(bytes) : "memory");
+}
+// bounded
+__device__ __forceinline__ void wait(uint64_t* m, uint32_t parity, bool& failed, int* err) {
+  for (int it = 0; !failed; ++it) {
+    uint32_t ok;
+    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(ok) : "r"(su32(m)), "r"(parity) : "memory");
+    if (ok) return;
+    if (it >= WAIT_LIMIT) {
+      failed = true;
+      if (err) atomicOr(err, 8);
+    }
+  }
+}
 
 __global__ void __launch_bounds__(NT, 1) chain_kernel(const __grid_constant__ ChainParams P) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -74,7 +97,7 @@ __global__ void __launch_bounds__(NT, 1) chain_kernel(const __grid_constant__ Ch
     if (pk == na) return;
     const int L = rows(pk), n = min(ROWS / L, last(pk) - pcol);
     const uint32_t bar = su32(&S.full[issued % NSLOT]), bytes = (uint32_t)(n * L * sizeof(cd));
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+    expect(&S.full[issued % NSLOT], bytes);
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
                      "r"(su32(S.ring[issued % NSLOT])), "l"(P.B + poff + (int64_t)pcol * L), "r"(bytes), "r"(bar) : "memory");
     pcol += n;
@@ -82,7 +105,9 @@ __global__ void __launch_bounds__(NT, 1) chain_kernel(const __grid_constant__ Ch
   };
   if (tid == 0) {
     for (int i = 0; i < NSLOT; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(su32(&S.full[i])) : "memory");
+    for (int i = 0; i < 2; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(su32(&S.vfull[i])) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    for (int j = 1; j <= 2 && j < na; ++j) expect(&S.vfull[j & 1], (uint32_t)(P.dims[j] * sizeof(cd)));
     for (int i = 0; i < NSLOT; ++i) issue();
     S.v[0][0] = cmk(1.0, 0.0);
   }
@@ -92,66 +117,83 @@ __global__ void __launch_bounds__(NT, 1) chain_kernel(const __grid_constant__ Ch
   }
   cluster.sync();
 
-  int used = 0;   // ring slots consumed
+  // An entry of v_{k+1} to rank q (the last bond is 1 and goes out).  A peer's v_{k+2} overwrites v_k
+  // after it has all of v_{k+1}, so after this CTA has read v_k, and u and the ring of site k.
+  auto push = [&](int k, int col, cd x, int q) {
+    if (k + 1 == na) {
+      if (q == 0) *P.out = x;
+      return;
+    }
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::
+                     "r"(mapa(su32(&S.v[(k + 1) & 1][col]), q)), "l"(__double_as_longlong(x.x)), "l"(__double_as_longlong(x.y)),
+                     "r"(mapa(su32(&S.vfull[(k + 1) & 1]), q)) : "memory");
+  };
+  int used = 0, owed = 0;   // ring slots consumed; of these not yet refilled
   bool failed = false;
   for (int k = 0; k < na; ++k) {
-    const int L = rows(k), chiL = P.dims[k], c0 = first(k), c1 = last(k), per = ROWS / L;
-    if (c1 > c0) {
+    const int L = rows(k), chiL = P.dims[k], c0 = first(k), nb = last(k) - c0, per = ROWS / L;
+    if (k > 0) wait(&S.vfull[k & 1], (uint32_t)((k - 1) >> 1) & 1, failed, P.err);
+    if (nb > 0) {
       const cd* v = S.v[k & 1];
       for (int a = tid; a < chiL; a += NT) {
         const cd x = v[a];
         for (int s = 0; s < d; ++s) S.u[s * chiL + a] = cmul(x, S.f[k * d + s]);
       }
-      __syncthreads();
     }
-    // warps per column: all eight when a slot holds one, one when it holds eight or more
-    const int lw = per >= 8 ? 0 : (per >= 4 ? 1 : (per >= 2 ? 2 : 3)), wpc = 1 << lw, wsub = warp & (wpc - 1);
-    for (int col = c0; col < c1; col += per, ++used) {
-      const int n = min(per, c1 - col);
-      const uint32_t bar = su32(&S.full[used % NSLOT]);
-      for (int it = 0; !failed; ++it) {   // bounded
-        uint32_t ok;
-        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-                     : "=r"(ok) : "r"(bar), "r"((uint32_t)(used / NSLOT) & 1) : "memory");
-        if (ok) break;
-        if (it >= WAIT_LIMIT) {
-          failed = true;
-          if (P.err) atomicOr(P.err, 8);
-        }
+    __syncthreads();
+    if (tid == 0 && !failed) {
+      if (k > 0 && k + 2 < na) expect(&S.vfull[k & 1], (uint32_t)(P.dims[k + 2] * sizeof(cd)));
+      for (int i = 0; i < owed; ++i) issue();
+    }
+    owed = 0;
+    const int slots = (nb + per - 1) / per;
+    auto dot = [&](const cd* b, int r, int step) {   // this warp's part of a column: rows r, r + step, ...
+      cd s0 = cmk(0.0, 0.0), s1 = cmk(0.0, 0.0);
+      for (; r + step < L; r += 2 * step) {
+        cfma(s0, S.u[r], b[r]);
+        cfma(s1, S.u[r + step], b[r + step]);
       }
-      for (int j = warp >> lw; j < n; j += NW >> lw) {
-        const cd* b = S.ring[used % NSLOT] + j * L;
-        cd s0 = cmk(0.0, 0.0), s1 = cmk(0.0, 0.0);
-        int r = wsub * 32 + lane;
-        for (; r + 32 * wpc < L; r += 64 * wpc) {
-          cfma(s0, S.u[r], b[r]);
-          cfma(s1, S.u[r + 32 * wpc], b[r + 32 * wpc]);
-        }
-        if (r < L) cfma(s0, S.u[r], b[r]);
-        cd s = cadd(s0, s1);
+      if (r < L) cfma(s0, S.u[r], b[r]);
+      cd s = cadd(s0, s1);
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-          s.x += __shfl_xor_sync(0xffffffffu, s.x, off);
-          s.y += __shfl_xor_sync(0xffffffffu, s.y, off);
-        }
-        if (lane == 0) S.part[col - c0 + j][wsub] = s;
+      for (int off = 16; off > 0; off >>= 1) {
+        s.x += __shfl_xor_sync(0xffffffffu, s.x, off);
+        s.y += __shfl_xor_sync(0xffffffffu, s.y, off);
       }
-      __syncthreads();   // the slot is consumed
-      if (tid == 0 && !failed) issue();
-    }
-    // this CTA's entries of v' to every CTA
-    const int nb = c1 - c0;
-    {
-      const int q = tid / (NT / C);   // sixteen threads per rank
-      for (int j = tid % (NT / C); j < nb; j += NT / C) {
+      return s;
+    };
+    if (slots <= NSLOT / 2) {
+      // a warp per column, which pushes it; the slots are refilled at the next site
+      for (int j = warp; j < nb; j += NW) {
+        const int sl = used + j / per;
+        wait(&S.full[sl % NSLOT], (uint32_t)(sl / NSLOT) & 1, failed, P.err);
+        const cd s = dot(S.ring[sl % NSLOT] + (j % per) * L, lane, 32);
+        if (lane < C) push(k, c0 + j, s, lane);
+      }
+      used += slots;
+      owed = slots;
+    } else {
+      // slot by slot, each refilled when it is consumed; warps per column: all eight when a slot holds
+      // one, one when it holds eight or more
+      const int lw = per >= 8 ? 0 : (per >= 4 ? 1 : (per >= 2 ? 2 : 3)), wpc = 1 << lw, wsub = warp & (wpc - 1);
+      for (int col = 0; col < nb; col += per, ++used) {
+        const int n = min(per, nb - col);
+        wait(&S.full[used % NSLOT], (uint32_t)(used / NSLOT) & 1, failed, P.err);
+        for (int j = warp >> lw; j < n; j += NW >> lw) {
+          const cd s = dot(S.ring[used % NSLOT] + j * L, wsub * 32 + lane, 32 * wpc);
+          if (lane == 0) S.part[col + j][wsub] = s;
+        }
+        __syncthreads();   // the slot is consumed
+        if (tid == 0 && !failed) issue();
+      }
+      for (int j = tid % (NT / C); j < nb; j += NT / C) {   // sixteen threads per rank
         cd s = S.part[j][0];
         for (int w = 1; w < wpc; ++w) s = cadd(s, S.part[j][w]);
-        *cluster.map_shared_rank(&S.v[(k + 1) & 1][c0 + j], q) = s;
-        if (k == na - 1 && q == 0) *P.out = s;   // the last bond is 1
+        push(k, c0 + j, s, tid / (NT / C));
       }
     }
-    cluster.sync();
   }
+  cluster.sync();
   if (failed && tid == 0)   // let the copies in flight land (bounded) before the CTA goes away
     for (int i = 0; i < WAIT_LIMIT && i >= 0; ++i) __nanosleep(1);
 }
