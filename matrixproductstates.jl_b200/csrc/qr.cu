@@ -54,7 +54,7 @@
 // SMs.  One row per lane and many CTAs beat more rows per lane (512 x 128 at 1 / 2 / 4 rows: 254 / 324
 // / 491 us) because the products scale with the CTAs.
 // Against the form with a reflector warp behind block barriers, Q as GEMMs over a back substitution
-// and outer panels of 16 columns (B200, Q only): 64 x 32 108.7 -> 47.6 us, 512 x 128 394 -> 235,
+// and outer panels of 16 columns (B200, Q only): 64 x 32 108.7 -> 45.6 us, 512 x 128 394 -> 235,
 // 512 x 256 818 -> 590, 2048 x 512 3990 -> 2090.
 #include <cooperative_groups.h>
 
@@ -884,7 +884,10 @@ struct Choice {
   size_t smem = 0;
 };
 
-// Cluster of C = ceil(m / (32 rpl)) CTAs, at most 16: prefer 1 row per lane, then 2, then 4; the
+// Cluster of C = ceil(m / (32 rpl)) CTAs, at most 16: prefer 1 row per lane, then 2, then 4, since the
+// products scale with the CTAs -- except 33 to 64 rows of up to 32 columns, where two rows per lane in
+// one CTA save the exchanges (48 x 24: 40.6 -> 39.4 us, 64 x 32: 47.6 -> 45.6; but 64 x 64: 98.8 ->
+// 100.9, 128 x 32 in two CTAs: 47.7 -> 53.8, 200 x 100: 177 -> 216).  The
 // widest column chunk of the block reflectors that fits, in steps of 8 (512 x 256, one width against
 // the next: 88 columns 635 us, 64 columns 675, as a chunk costs about 3500 clocks of exchanges
 // whatever its width).  An outer panel of the blocked form
@@ -894,6 +897,7 @@ bool choose(int m, int n, Choice& ch, bool panel = false) {
   const int nc_max = panel ? std::max(8, (n - NB + 7) / 8 * 8) : std::min(256, (n + 7) / 8 * 8);
   const int nc_min = panel ? nc_max : 8;
   for (int rpl : {1, 2, 4}) {
+    if (rpl == 1 && m > 32 && m <= 64 && n <= 32) continue;
     const int rows = 32 * rpl;
     const int C = (m + rows - 1) / rows;
     if (C > CMAX) continue;
